@@ -6,7 +6,8 @@
 //           s+1 runs while the warpgroup works on step s.  With 64-wide KV blocks and
 //           a two-stage ring two such CTAs share an SM.
 //   NT = 1, AW = 2  the same tile with two softmax warpgroups that take the KV steps
-//           in turn (128-wide KV blocks).  The groups hand the stale row maximum to
+//           in turn (128-wide KV blocks; 64-wide ones at head_dim_v 64, still two CTAs
+//           per SM, and above 128).  The groups hand the stale row maximum to
 //           one another through shared memory, keep partial row sums and split the
 //           epilogue; P has tensor-memory columns of its own, so the S buffer of step
 //           s is free as soon as its softmax has read it and Q.K^T of step s+2 runs
@@ -100,17 +101,20 @@ struct FwdLayout {
   static constexpr int kOCol = AW == 2 ? 3 * BKV : 2 * BKV;
   static constexpr int kTmemUsed = kOCol + NT * DV;
   static constexpr int kTmemCols = kTmemUsed <= 128 ? 128 : (kTmemUsed <= 256 ? 256 : 512);
-  static_assert(kTmemUsed <= 512, "tensor memory has 512 columns");
+  // CTAs that share an SM: the launch bound that keeps their registers within the file.
+  static constexpr int kCtasPerSm = (NT == 1 && BKV == 64 && D <= 128 && DV <= 128) ? 2 : 1;
+  static_assert(kTmemCols <= 512 / kCtasPerSm, "tensor memory has 512 columns per SM");
   static constexpr int kSoftmaxGroups = NT * AW;
   static constexpr int kThreads = (kSoftmaxGroups + 1) * 128;
   // Row maxima shared by the alternating warpgroups, and their partial row sums.
   static constexpr int kShareBytes = AW > 1 ? 3 * kTile * 4 : 0;
   static constexpr bool kOStageInQ = (NT == 2) || (DV <= D);
   // Register split between the warpgroups when there are two softmax warpgroups
-  // (multiples of 8; 2 * 128 * softmax + 128 * producer <= 64K).
+  // (multiples of 8).  One CTA per SM starts with 168 registers a thread: 384 * 168 = 256 * 216 +
+  // 128 * 72; two start with 80 each: 384 * 80 = 256 * 104 + 128 * 32.
   static constexpr bool kSplitRegs = kSoftmaxGroups == 2;
-  static constexpr int kSoftmaxRegs = 216;
-  static constexpr int kProducerRegs = 72;
+  static constexpr int kSoftmaxRegs = kCtasPerSm == 2 ? 104 : 216;
+  static constexpr int kProducerRegs = kCtasPerSm == 2 ? 32 : 72;
 
   // `list_steps`: capacity of the list of steps that survive segment skipping (0 = no list).
   __host__ __device__ static size_t smem_bytes(int stages, bool dense, bool seg, int list_steps = 0) {
@@ -150,7 +154,7 @@ struct FwdBarriers {
 // PLAIN: no soft-cap, no segment ids, no streamed mask blocks -- those blocks of the
 // softmax loop are compiled out, which shortens the instruction stream of the common case.
 template <int D, int DV, int BKV, int NT, int AW, bool PLAIN, bool BF16>
-__global__ void __launch_bounds__((NT * AW + 1) * 128, 1)
+__global__ void __launch_bounds__((NT * AW + 1) * 128, (FwdLayout<D, DV, BKV, NT, AW>::kCtasPerSm))
 splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                   const FwdArgs a) {

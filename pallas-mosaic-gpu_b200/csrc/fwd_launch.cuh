@@ -3,8 +3,6 @@
 // the kernel for a given (head_dim, head_dim_v, block_kv, tiles) combination.
 #pragma once
 
-#include <cstdlib>
-
 #include "dispatch.h"
 #include "fwd_kernel.cuh"
 #include "host_common.cuh"
@@ -87,29 +85,26 @@ int launch_fwd_typed(const SplashParams& p, cudaStream_t stream) {
   return launch_fwd_plain<D, DV, BKV, NT, AW, false, BF16>(p, stream);
 }
 
-// Softmax warpgroups that alternate over the KV steps of a one-tile kernel;
-// SPLASH_FWD_AW=1|2 overrides the default (experiments).
-inline int fwd_alternating_groups() {
-  static const int forced = [] {
-    const char* e = getenv("SPLASH_FWD_AW");
-    return e ? atoi(e) : 0;
-  }();
-  return (forced == 1 || forced == 2) ? forced : 2;
+// Softmax warpgroups per q tile of the one-tile kernel.  Two that alternate over the KV steps where
+// tensor memory has room for P beside S: 128-wide blocks always (causal, 16 heads, seq 8192, D = 128:
+// 449 us against 532 with one group), 64-wide blocks where the softmax bounds the step (two CTAs per SM,
+// D = 64, 64 heads, seq 8192 causal: 742 against 786 us; packed documents 734 against 750) or a step is
+// long enough for its latency to show (one CTA per SM, D = 256, 64 heads, block-sparse seq 8192: 1092
+// against 1145 us; D = 192: 348 against 356).  At DV = 128 with 64-wide blocks P lies over S in the 256
+// columns each of two CTAs has, and one group is better (causal seq 8192: 457 against 490 us).
+template <int DV, int BKV, int NT>
+constexpr int fwd_softmax_groups() {
+  if (NT == 2) return 1;
+  if (BKV == 64) return (DV == 64 || DV > 128) ? 2 : 1;
+  return 3 * BKV + DV <= 512 ? 2 : 1;
 }
 
 template <int D, int DV, int BKV, int NT>
 int launch_fwd(const SplashParams& p, cudaStream_t stream) {
   const bool bf16 = p.dtype == SPLASH_DTYPE_BF16;
-  // Two alternating groups with 128-column blocks; with 64-column blocks one group
-  // keeps the kernel small enough for two CTAs per SM, which serves that tiling better.
-  if constexpr (NT == 1 && BKV == 128 && 3 * BKV + DV <= 512) {
-    if (fwd_alternating_groups() == 2) {
-      if (bf16) return launch_fwd_typed<D, DV, BKV, NT, 2, true>(p, stream);
-      return launch_fwd_typed<D, DV, BKV, NT, 2, false>(p, stream);
-    }
-  }
-  if (bf16) return launch_fwd_typed<D, DV, BKV, NT, 1, true>(p, stream);
-  return launch_fwd_typed<D, DV, BKV, NT, 1, false>(p, stream);
+  constexpr int AW = fwd_softmax_groups<DV, BKV, NT>();
+  if (bf16) return launch_fwd_typed<D, DV, BKV, NT, AW, true>(p, stream);
+  return launch_fwd_typed<D, DV, BKV, NT, AW, false>(p, stream);
 }
 
 }  // namespace splash
