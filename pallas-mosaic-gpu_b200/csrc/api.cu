@@ -1,7 +1,5 @@
 // extern "C" entry points of libsplash_sm100.so: argument validation, dispatch to
 // the compiled kernel configuration, status helpers.
-#include <cstdlib>
-
 #include "dispatch.h"
 #include "host_common.cuh"
 
@@ -133,8 +131,8 @@ extern "C" int splash_bwd_dkv(const SplashParams* p, void* stream) {
   if (int rc = launch_seg_ranges(*p, st)) return rc;
   // The kernel works in steps of 64 q rows with double-buffered scores; `sub_block`
   // is accepted for compatibility and does not change the tiling.
-  if (p->head_dim == 64) return p->head_dim_v == 64 ? launch_bwd_col<64, 64, false>(*p, st) : launch_bwd_col<64, 128, false>(*p, st);
-  return p->head_dim_v == 128 ? launch_bwd_col<128, 128, false>(*p, st) : launch_bwd_col<128, 64, false>(*p, st);
+  if (p->head_dim == 64) return p->head_dim_v == 64 ? launch_bwd_col<64, 64>(*p, st) : launch_bwd_col<64, 128>(*p, st);
+  return p->head_dim_v == 128 ? launch_bwd_col<128, 128>(*p, st) : launch_bwd_col<128, 64>(*p, st);
 }
 
 // The f32 dQ accumulator alone.
@@ -162,14 +160,7 @@ extern "C" int splash_bwd_fused(const SplashParams* p, void* stream) {
   } else {
     SPLASH_CUDA_CHECK(cudaMemsetAsync(p->dq_acc, 0, static_cast<size_t>(dq_acc_bytes(p)), st));
   }
-  // Head dim 128 takes the kernel that works on whole 128-row q blocks; streamed mask blocks
-  // and head dim 64 take the 64-row one.  SPLASH_BWD_WIDE=0 forces the latter (experiments).
-  const char* wide_env = getenv("SPLASH_BWD_WIDE");
-  const bool wide_off = wide_env && wide_env[0] == '0';
-  int rc;
-  if (!wide_off && bwd_wide_supported(*p)) rc = launch_bwd_wide(*p, st);
-  else rc = p->head_dim == 64 ? launch_bwd_col<64, 64, true>(*p, st) : launch_bwd_col<128, 128, true>(*p, st);
-  if (rc) return rc;
+  if (int rc = launch_bwd_wide(*p, st)) return rc;
   return launch_dq_transpose_cast(p->dq_acc, p->dq, static_cast<long long>(p->batch) * p->heads, p->head_dim, p->q_len,
                                   p->dtype, st);
 }

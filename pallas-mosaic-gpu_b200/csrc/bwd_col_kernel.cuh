@@ -4,10 +4,7 @@
 // sees it, for every q head of the KV head's group, so dK and dV are complete when
 // the CTA ends: GQA/MQA heads are reduced in tensor memory, not across CTAs.
 //
-//   FUSED = false   dK, dV only (the split backward; dQ comes from bwd_row_kernel).
-//   FUSED = true    also dQ: each step's dQ^T = K^T dS^T tile is reduce-added into an
-//                   f32 accumulator laid out [batch, heads, head_dim, q_len] with a
-//                   TMA add-reduction (64 q rows per step).
+// It computes dK and dV of the split backward; dQ comes from bwd_row_kernel.
 //
 // Per step (64 q rows of one q block):
 //   S^T  = K Q^T        smem x smem -> TMEM f32   [128 kv, 64]
@@ -15,19 +12,16 @@
 //   elementwise (thread = kv row, two warpgroups split the 64 columns):
 //     P^T  = exp2((S^T - lse) log2e)   masked entries 0
 //     dS^T = P^T (dP^T - delta) [ (1 - tanh^2) with soft-cap ]
-//     both written back over the columns they came from as packed 16-bit; FUSED also
-//     stages dS^T in shared memory
+//     both written back over the columns they came from as packed 16-bit
 //   dV  += P^T dO       TMEM x smem
 //   dK  += dS^T Q       TMEM x smem
-//   dQ^T = K^T dS^T     smem x smem (FUSED), written over the dead dP^T columns and
-//                       drained by a writer warpgroup
 //
 // S^T and dP^T are double-buffered in tensor memory: the scores of step t+2 are issued
 // while the elementwise warps work on step t+1, so the tensor core and the elementwise
 // warps overlap instead of taking turns.  That needs three Q/dO tiles in flight.
 //
-// Behaviour follows the reference kernels (splash_attention_mgpu/backward.py:377-785,
-// backward_fused.py:64-512); the code shares nothing with them.
+// Behaviour follows the reference kernel (splash_attention_mgpu/backward.py:377-785); the
+// code shares nothing with it.
 #pragma once
 
 #include <stddef.h>
@@ -67,50 +61,40 @@ struct BwdArgs {
 };
 
 enum BwdSite : int {
-  kBSiteTmaEmpty = 21, kBSiteMmaKV, kBSiteMmaFull, kBSiteMmaP, kBSiteMmaDqFree,
-  kBSiteEwFull, kBSiteEwS, kBSiteEwDone, kBSiteEwEpi,
-  kBSiteWrReady, kBSiteWrBarA, kBSiteWrBarB,
+  kBSiteTmaEmpty = 21, kBSiteMmaKV, kBSiteMmaFull, kBSiteMmaP,
+  kBSiteEwFull = 26, kBSiteEwS, kBSiteEwDone, kBSiteEwEpi,
 };
 
 constexpr int kColBC = 64;  // q rows per step
 
-template <int D, int DV, bool FUSED>
+template <int D, int DV>
 struct ColLayout {
-  static_assert(!FUSED || D == DV, "the fused kernel needs head_dim == head_dim_v");
   static constexpr int kRows = 128;  // kv rows per CTA
   static constexpr int BC = kColBC;
   static constexpr int kSub = 128 / BC;
   static constexpr int kKBytes = kRows * D * 2;
   static constexpr int kVBytes = kRows * DV * 2;
-  // FUSED at head_dim 64: dQ^T = K^T dS^T is issued with M = 128 like at head_dim 128, and
-  // the second 64 rows of its A operand are a second copy of the K tile, so the upper half
-  // of the result repeats the lower half and is simply not stored.  That keeps one
-  // accumulator layout and one writer for both head dims at the price of idle MMA rows.
-  static constexpr int kKDupBytes = (FUSED && D == 64) ? kRows * 128 : 0;
   static constexpr int kQStage = BC * D * 2;
   static constexpr int kDoStage = BC * DV * 2;
   static constexpr int kVecStage = BC * 4;          // lse, delta, q segment ids: BC words each
   static constexpr int kMaskStage = kRows * 128 / 8;  // a whole transposed block, one bit per element
-  static constexpr int kDsStage = kRows * BC * 2;   // FUSED: dS^T as an MMA operand
-  static constexpr int kDqStage = 128 * 32 * 4;     // FUSED: half a dQ^T tile (32 q columns), f32
   // Tensor memory columns: two S^T buffers, two dP^T buffers, dK, dV.  P^T lives in the
-  // S^T buffer it came from, dS^T in the dP^T buffer, dQ^T reuses the dP^T buffer.
+  // S^T buffer it came from, dS^T in the dP^T buffer.
   static constexpr int kColS = 0, kColDp = 2 * BC, kColDk = 4 * BC, kColDv = 4 * BC + D;
   static constexpr int kTmemUsed = 4 * BC + D + DV;
   static constexpr int kTmemCols = 512;
   static constexpr int kEwThreads = 256;
-  static constexpr int kThreads = kEwThreads + (FUSED ? 128 : 0) + 128;
+  static constexpr int kThreads = kEwThreads + 128;
   static_assert(kTmemUsed <= 512, "tensor memory budget");
 
   // `list_steps`: capacity of the list of block steps that survive segment skipping (0 = no list).
   __host__ __device__ static size_t smem_bytes(int stages, bool dense, bool seg, int list_steps = 0) {
     size_t b = 1024;
     b += (static_cast<size_t>(list_steps) * 2 + 15) & ~static_cast<size_t>(15);
-    b += kKBytes + kKDupBytes + kVBytes;
+    b += kKBytes + kVBytes;
     b += static_cast<size_t>(stages) * (kQStage + kDoStage + 2 * kVecStage);
     if (seg) b += static_cast<size_t>(stages) * kVecStage;
     if (dense) b += static_cast<size_t>(stages) * kMaskStage;
-    if (FUSED) b += 2 * kDsStage + kDqStage;
     b += 1024;
     return b;
   }
@@ -122,7 +106,6 @@ struct ColBarriers {
   uint64_t kv_full;
   uint64_t full[kBwdMaxStages], empty[kBwdMaxStages];
   uint64_t s_ready[2], p_ready[2], acc_done;
-  uint64_t dq_ready, dq_free, wr_a, wr_b;
   uint64_t epi[2];
   uint32_t tmem_base;
   uint32_t abort_flag;
@@ -192,19 +175,18 @@ struct ColSteps {
 };
 
 // PLAIN: no soft-cap, no segment ids, no streamed mask blocks -- that code is compiled out.
-template <int D, int DV, bool FUSED, bool PLAIN, bool BF16>
-__global__ void __launch_bounds__(ColLayout<D, DV, FUSED>::kThreads, 1)
+template <int D, int DV, bool PLAIN, bool BF16>
+__global__ void __launch_bounds__(ColLayout<D, DV>::kThreads, 1)
 splash_bwd_col_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                       const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
-                      const __grid_constant__ CUtensorMap tm_dqacc, const BwdArgs a) {
-  using L = ColLayout<D, DV, FUSED>;
+                      const BwdArgs a) {
+  using L = ColLayout<D, DV>;
   constexpr int kRows = 128;
   constexpr int BC = kColBC;
   constexpr int kSub = L::kSub;
   constexpr int kEwWarps = 8;
-  constexpr int kWriterWarp0 = kEwWarps;                       // FUSED only
-  constexpr int kProducerWarp0 = kEwWarps + (FUSED ? 4 : 0);
+  constexpr int kProducerWarp0 = kEwWarps;
 
   const bool has_dense = !PLAIN && a.has_dense;
   const bool has_seg = !PLAIN && a.has_seg;
@@ -212,12 +194,10 @@ splash_bwd_col_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   extern __shared__ uint8_t smem_raw[];
   const int stages = a.stages;
   const uint32_t k_u32 = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t v_u32 = k_u32 + L::kKBytes + L::kKDupBytes;
+  const uint32_t v_u32 = k_u32 + L::kKBytes;
   const uint32_t q_u32 = v_u32 + L::kVBytes;
   const uint32_t do_u32 = q_u32 + stages * L::kQStage;
-  const uint32_t ds_u32 = do_u32 + stages * L::kDoStage;              // FUSED: 2 x dS^T
-  const uint32_t dqs_u32 = ds_u32 + (FUSED ? 2 * L::kDsStage : 0);    // FUSED: dQ^T staging
-  const uint32_t mask_u32 = dqs_u32 + (FUSED ? L::kDqStage : 0);
+  const uint32_t mask_u32 = do_u32 + stages * L::kDoStage;
   const uint32_t lse_u32 = mask_u32 + (has_dense ? stages * L::kMaskStage : 0);
   const uint32_t delta_u32 = lse_u32 + stages * L::kVecStage;
   const uint32_t segq_u32 = delta_u32 + stages * L::kVecStage;
@@ -258,7 +238,7 @@ splash_bwd_col_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       uint32_t count = 1;
       if (off >= offsetof(ColBarriers, empty) && off < offsetof(ColBarriers, s_ready)) count = 1 + kEwWarps;
       if (off >= offsetof(ColBarriers, p_ready) && off < offsetof(ColBarriers, acc_done)) count = L::kEwThreads;
-      if (off >= offsetof(ColBarriers, dq_free) && off < offsetof(ColBarriers, tmem_base)) count = 128;  // dq_free, wr_a, wr_b, epi
+      if (off >= offsetof(ColBarriers, epi)) count = 128;
       mbar_init(bars_u32 + off, count);
     }
     if (lane == 0) {
@@ -304,11 +284,10 @@ splash_bwd_col_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       if (elect_one()) {
         prefetch_tensormap(&tm_q);
         prefetch_tensormap(&tm_do);
-        mbar_arrive_expect_tx(SPLASH_CBAR(kv_full, 0), L::kKBytes + L::kKDupBytes + L::kVBytes);
+        mbar_arrive_expect_tx(SPLASH_CBAR(kv_full, 0), L::kKBytes + L::kVBytes);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c)
           tma_load_2d(k_u32 + c * (kRows * 128), &tm_k, c * 64, kv_row0, SPLASH_CBAR(kv_full, 0));
-        if constexpr (L::kKDupBytes > 0) tma_load_2d(k_u32 + L::kKBytes, &tm_k, 0, kv_row0, SPLASH_CBAR(kv_full, 0));
 #pragma unroll
         for (int c = 0; c < DV / 64; ++c)
           tma_load_2d(v_u32 + c * (kRows * 128), &tm_v, c * 64, kv_row0, SPLASH_CBAR(kv_full, 0));
@@ -349,7 +328,6 @@ splash_bwd_col_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       constexpr uint32_t kIdescScore = make_idesc(BF16, 128, BC, false, false);   // K Q^T, V dO^T
       constexpr uint32_t kIdescAcc = make_idesc(BF16, 128, D, false, true);       // dS^T Q
       constexpr uint32_t kIdescAccV = make_idesc(BF16, 128, DV, false, true);     // P^T dO
-      constexpr uint32_t kIdescDq = make_idesc(BF16, 128, BC, true, true);        // K^T dS^T
       auto issue_s = [&](int slot, int buf) {
         const uint32_t k_lo = desc_lo(k_u32, 16), q_lo = desc_lo(q_u32 + slot * L::kQStage, 16);
 #pragma unroll
@@ -395,20 +373,6 @@ splash_bwd_col_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
               umma_ts2_w(tmem + L::kColDk, tmem + L::kColDp + buf * BC + (kk >> 1) * 32 + (kk & 1) * 8,
                          q_lo + ((kk * 2048) >> 4), kDescHi, kIdescAcc, (t > 0 || kk > 0) ? 1u : 0u);
           }
-          if constexpr (FUSED) {
-            // dQ^T[d, q] = sum_kv K[kv, d] dS^T[kv, q]: A = K read MN-major, B = staged dS^T
-            // MN-major.  The result replaces dP^T / dS^T of this step, which dK has consumed
-            // (the tensor core runs its instructions in issue order).  It is issued this
-            // early so that the writer has drained it long before the next dP^T needs the
-            // columns.
-            const uint32_t k_lo = desc_lo(k_u32, kRows * 128);
-            const uint32_t ds_lo = desc_lo(ds_u32 + buf * L::kDsStage, kRows * 128);
-#pragma unroll
-            for (int kk = 0; kk < kRows / 16; ++kk)
-              umma_ss2_w(tmem + L::kColDp + buf * BC, k_lo + ((kk * 2048) >> 4), kDescHi, ds_lo + ((kk * 2048) >> 4),
-                         kDescHi, kIdescDq, kk > 0);
-            umma_commit_w(SPLASH_CBAR(dq_ready, 0));
-          }
           {
             // dV += P^T dO
             const uint32_t do_lo = desc_lo(do_u32 + c_slot * L::kDoStage, BC * 128);
@@ -423,69 +387,14 @@ splash_bwd_col_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             if (!warp_wait(SPLASH_CBAR(full, s_slot), s_phase, ctx, kBSiteMmaFull, t + 2)) break;
             tc_fence_after();
             issue_s(s_slot, buf);
-            if constexpr (FUSED) {
-              // The writer must have taken dQ^T of step t out of the dP^T buffer.
-              if (!warp_wait(SPLASH_CBAR(dq_free, 0), t & 1, ctx, kBSiteMmaDqFree, t)) break;
-              tc_fence_after();
-            }
             issue_dp(s_slot, buf);
             umma_commit_w(SPLASH_CBAR(s_ready, buf));
             if (++s_slot == stages) { s_slot = 0; s_phase ^= 1; }
-          } else if constexpr (FUSED) {
-            // Tail steps: still observe every phase of dq_free, so that dq_ready never
-            // runs two phases ahead of the writer.
-            if (!warp_wait(SPLASH_CBAR(dq_free, 0), t & 1, ctx, kBSiteMmaDqFree, t)) break;
           }
           if (++c_slot == stages) c_slot = 0;
         }
         umma_commit_w(SPLASH_CBAR(acc_done, 0));
       }
-    }
-  } else if (FUSED && warp >= kWriterWarp0) {
-    // ================================ dQ writer ==================================
-    if constexpr (FUSED) {
-      const int wq = warp & 3;
-      const int drow = wq * 32 + lane;  // head-dim index = TMEM lane
-      const uint32_t dq_tmem = tmem + (static_cast<uint32_t>(wq * 32) << 16) + L::kColDp;
-      const bool leader = (warp == kWriterWarp0 && lane == 0);
-      bool alive = true;
-      int t = 0;
-      for (; it.valid() && alive; it.next(), ++t) {
-        const int qblk = a.block_list[it.off()];
-        if (!warp_wait(SPLASH_CBAR(dq_ready, 0), t & 1, ctx, kBSiteWrReady, t)) break;
-        tc_fence_after();
-        uint32_t acc[BC];
-#pragma unroll
-        for (int c = 0; c < BC / 32; ++c) tmem_ld32(dq_tmem + (t & 1) * BC + c * 32, acc + c * 32);
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(SPLASH_CBAR(dq_free, 0));
-        const int x = qblk * 128 + it.sb * BC;
-        const int y = (b * a.heads + it.head()) * D;
-        // Two passes of 32 q columns through one 16 KB staging tile (128 rows of 128 bytes).
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const uint32_t par = (2 * t + half) & 1;
-          // The previous reduction must have read the staging tile.
-          if (leader) bulk_wait_group_read<0>();
-          mbar_arrive(SPLASH_CBAR(wr_a, 0));
-          if (!warp_wait(SPLASH_CBAR(wr_a, 0), par, ctx, kBSiteWrBarA, t)) { alive = false; break; }
-          if (drow < D) {  // at head_dim 64 the upper rows repeat the lower ones
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-              sts128(dqs_u32 + swz128(drow, c), make_uint4(acc[half * 32 + c * 4], acc[half * 32 + c * 4 + 1],
-                                                           acc[half * 32 + c * 4 + 2], acc[half * 32 + c * 4 + 3]));
-          }
-          fence_proxy_async_smem();
-          mbar_arrive(SPLASH_CBAR(wr_b, 0));
-          if (!warp_wait(SPLASH_CBAR(wr_b, 0), par, ctx, kBSiteWrBarB, t)) { alive = false; break; }
-          if (leader) {
-            tma_reduce_add_2d(&tm_dqacc, dqs_u32, x + half * 32, y);
-            bulk_commit_group();
-          }
-        }
-      }
-      if (leader) bulk_wait_group_read<0>();
     }
   } else {
     // ========================== elementwise warpgroups ===========================
@@ -624,21 +533,11 @@ splash_bwd_col_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           // Packed results go over the first half of the columns this thread just read.
           tmem_st16(tmem_row + L::kColS + buf * BC + col0, ppk);
           tmem_st16(tmem_row + L::kColDp + buf * BC + col0, dspk);
-          if constexpr (FUSED) {
-            // dS^T staged as [kv row][64 q], 128 bytes per row, 128-byte swizzle.
-            const uint32_t stage = ds_u32 + buf * L::kDsStage;
-            const int chunk0 = (col0 + c * 32) / 8;  // 16-byte chunk index of this thread's first column
-#pragma unroll
-            for (int g = 0; g < 4; ++g)
-              sts128(stage + swz128(row, chunk0 + g),
-                     make_uint4(dspk[g * 4], dspk[g * 4 + 1], dspk[g * 4 + 2], dspk[g * 4 + 3]));
-          }
         }
         // The slot's vectors and mask slice have been read.
         __syncwarp();
         if (lane == 0) mbar_arrive(SPLASH_CBAR(empty, slot));
         tmem_wait_st();
-        if constexpr (FUSED) fence_proxy_async_smem();
         tc_fence_before();
         mbar_arrive(SPLASH_CBAR(p_ready, buf));
         if (++slot == stages) { slot = 0; phase ^= 1; }

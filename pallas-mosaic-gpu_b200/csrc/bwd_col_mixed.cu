@@ -2,8 +2,8 @@
 // (see bwd_launch.cuh): dK/dV over the column schedule and dQ over the row schedule.
 #include "bwd_launch.cuh"
 namespace splash {
-template int launch_bwd_col<128, 64, false>(const SplashParams&, cudaStream_t);
-template int launch_bwd_col<64, 128, false>(const SplashParams&, cudaStream_t);
+template int launch_bwd_col<128, 64>(const SplashParams&, cudaStream_t);
+template int launch_bwd_col<64, 128>(const SplashParams&, cudaStream_t);
 template int launch_bwd_row<128, 64, 64>(const SplashParams&, cudaStream_t);
 template int launch_bwd_row<128, 64, 128>(const SplashParams&, cudaStream_t);
 template int launch_bwd_row<64, 128, 64>(const SplashParams&, cudaStream_t);

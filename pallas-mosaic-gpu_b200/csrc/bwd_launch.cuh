@@ -45,9 +45,9 @@ inline void fill_bwd_args(BwdArgs& a, const SplashParams& p, bool dense, bool se
   a.soft_cap = p.soft_cap;
 }
 
-template <int D, int DV, bool FUSED, bool BF16>
+template <int D, int DV, bool BF16>
 int launch_bwd_col_typed(const SplashParams& p, cudaStream_t stream) {
-  using L = ColLayout<D, DV, FUSED>;
+  using L = ColLayout<D, DV>;
   constexpr int BC = kColBC;
   const bool dense = p.partial_blocks != nullptr;
   const bool seg = p.seg_q != nullptr;
@@ -69,8 +69,7 @@ int launch_bwd_col_typed(const SplashParams& p, cudaStream_t stream) {
   const CUtensorMapDataType dt = tmap_dtype(p.dtype);
   const uint64_t q_rows = static_cast<uint64_t>(p.batch) * p.heads * p.q_len;
   const uint64_t kv_rows = static_cast<uint64_t>(p.batch) * p.kv_heads * p.kv_len;
-  CUtensorMap tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, tm_dqacc;
-  memset(&tm_dqacc, 0, sizeof tm_dqacc);
+  CUtensorMap tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv;
   if (dense && (reinterpret_cast<uintptr_t>(p.partial_blocks) & 15))
     return fail(SPLASH_INVALID_ARGUMENT, "partial_blocks not 16-byte aligned");
   int rc;
@@ -80,13 +79,6 @@ int launch_bwd_col_typed(const SplashParams& p, cudaStream_t stream) {
   if ((rc = make_tmap_2d(&tm_v, p.v, dt, 2, kv_rows, DV, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   if ((rc = make_tmap_2d(&tm_dk, p.dk, dt, 2, kv_rows, D, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   if ((rc = make_tmap_2d(&tm_dv, p.dv, dt, 2, kv_rows, DV, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
-  if (FUSED) {
-    // f32 accumulator viewed as [batch * heads * head_dim, q_len]; tiles of 32 q columns.
-    const uint64_t acc_rows = static_cast<uint64_t>(p.batch) * p.heads * D;
-    if ((rc = make_tmap_2d(&tm_dqacc, p.dq_acc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, acc_rows, p.q_len, D, 32,
-                           CU_TENSOR_MAP_SWIZZLE_128B)))
-      return rc;
-  }
   BwdArgs a;
   fill_bwd_args(a, p, dense, seg);
   a.stages = stages;
@@ -94,18 +86,18 @@ int launch_bwd_col_typed(const SplashParams& p, cudaStream_t stream) {
   a.seg_kv_ranges = skipping ? seg_kv_ranges(p) : nullptr;
   // The kernel without its soft-cap, segment and streamed-mask code when the call uses none.
   const bool plain = p.soft_cap == 0.f && !seg && !dense;
-  auto kernel = plain ? splash_bwd_col_kernel<D, DV, FUSED, true, BF16> : splash_bwd_col_kernel<D, DV, FUSED, false, BF16>;
+  auto kernel = plain ? splash_bwd_col_kernel<D, DV, true, BF16> : splash_bwd_col_kernel<D, DV, false, BF16>;
   if ((rc = opt_in_smem(kernel, smem))) return rc;
   const unsigned grid = static_cast<unsigned>(a.kv_blocks) * p.kv_heads * p.batch;
-  kernel<<<grid, L::kThreads, smem, stream>>>(tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, tm_dqacc, a);
+  kernel<<<grid, L::kThreads, smem, stream>>>(tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, a);
   SPLASH_CUDA_CHECK(cudaGetLastError());
   return SPLASH_OK;
 }
 
-template <int D, int DV, bool FUSED>
+template <int D, int DV>
 int launch_bwd_col(const SplashParams& p, cudaStream_t stream) {
-  if (p.dtype == SPLASH_DTYPE_BF16) return launch_bwd_col_typed<D, DV, FUSED, true>(p, stream);
-  return launch_bwd_col_typed<D, DV, FUSED, false>(p, stream);
+  if (p.dtype == SPLASH_DTYPE_BF16) return launch_bwd_col_typed<D, DV, true>(p, stream);
+  return launch_bwd_col_typed<D, DV, false>(p, stream);
 }
 
 template <int D, int DV, int BC>

@@ -5,10 +5,6 @@
 
 namespace splash {
 
-bool bwd_wide_supported(const SplashParams& p) {
-  return (p.head_dim == 128 || p.head_dim == 64) && p.head_dim_v == p.head_dim && p.partial_blocks == nullptr;
-}
-
 template <int D, bool BF16>
 static int launch_bwd_wide_typed(const SplashParams& p, cudaStream_t stream) {
   using L = WideLayout<D>;
@@ -29,8 +25,10 @@ static int launch_bwd_wide_typed(const SplashParams& p, cudaStream_t stream) {
   if ((rc = make_tmap_2d(&tm_dqacc, p.dq_acc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, acc_rows, p.q_len, 32, 32,
                          CU_TENSOR_MAP_SWIZZLE_128B)))
     return rc;
+  if (reinterpret_cast<uintptr_t>(p.partial_blocks) & 15)
+    return fail(SPLASH_INVALID_ARGUMENT, "partial_blocks not 16-byte aligned");
   BwdArgs a;
-  fill_bwd_args(a, p, false, seg);
+  fill_bwd_args(a, p, p.partial_blocks != nullptr, seg);
   a.stages = L::kSlots;
   if (L::kFold) {
     // The scratch holds the f32 dQ accumulator, then the folded -lse and -delta operands.
@@ -54,8 +52,8 @@ static int launch_bwd_wide_typed(const SplashParams& p, cudaStream_t stream) {
 }
 
 int launch_bwd_wide(const SplashParams& p, cudaStream_t stream) {
-  if (!bwd_wide_supported(p))
-    return fail(SPLASH_UNSUPPORTED, "the 128-row fused backward needs head_dim == head_dim_v in {64, 128} and no streamed mask blocks");
+  if (p.head_dim != p.head_dim_v || (p.head_dim != 64 && p.head_dim != 128))
+    return fail(SPLASH_UNSUPPORTED, "the fused backward needs head_dim == head_dim_v in {64, 128}");
   if (p.head_dim == 64) {
     if (p.dtype == SPLASH_DTYPE_BF16) return launch_bwd_wide_typed<64, true>(p, stream);
     return launch_bwd_wide_typed<64, false>(p, stream);

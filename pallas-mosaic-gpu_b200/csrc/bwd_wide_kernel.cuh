@@ -1,7 +1,7 @@
 // Splash attention fused backward over the column (per-KV-block) schedule with 128 q
-// rows per step, head_dim 128, sm_100a.
+// rows per step, head_dim 64 and 128, sm_100a.
 //
-// Why a second column kernel.  The 64-row-per-step kernel (bwd_col_kernel.cuh) is bound
+// Why whole q blocks.  A fused kernel in steps of 64 q rows (as bwd_col_kernel.cuh is) is bound
 // by the shared-memory data pipe, not by the tensor core: a tcgen05.mma that reads both
 // operands from shared memory streams M x 16 + N x 16 16-bit values per instruction, and
 // with N = 64 that is 6 KB for 32 cycles of arithmetic -- more than the 128 bytes per
@@ -119,8 +119,11 @@ static_assert(sizeof(WideBarriers) <= WideLayout<128>::kBarBytes, "barrier block
 #define SPLASH_WBAR(field, idx) \
   (bars_u32 + static_cast<uint32_t>(offsetof(WideBarriers, field)) + 8u * static_cast<uint32_t>(idx))
 
-// PLAIN: no soft-cap and no segment ids -- that code is compiled out.  Streamed (dense
-// int8) mask blocks are not handled here; calls that carry them take the 64-row kernel.
+// PLAIN: no soft-cap and no segment ids -- that code is compiled out.  The bits of a dense
+// partial block are read straight from global memory, 8 bytes per thread ahead of the step's
+// waits: 2 KB per block pair do not need a shared-memory ring, for which there is no room.
+// (Array mask, batch 2, 16/4 heads, seq 4096, D = 128: backward call 447 us in the 64-row kernel
+// with a ring, 357 us here.)
 template <int HEAD_DIM, bool PLAIN, bool BF16>
 __global__ void __launch_bounds__(WideLayout<HEAD_DIM>::kThreads, 1)
 splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -462,14 +465,23 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       int cur_mh = -1;
       int band_lo = -(1 << 30), band_hi = (1 << 30);  // allowed range of kv_pos - q_pos for this kv row
 
-      for (int t = 0; it.valid(); it.next(), ++t) {
+      int off_next = it.off();
+      int qblk_next = a.block_list[off_next], kind_next = a.block_kind[off_next];
+      for (int t = 0; t < total; ++t) {
         const int slot = t & 1;
         const uint32_t par = t & 1;
-        const int off = it.off();
-        const int qblk = a.block_list[off];
-        const bool partial = a.block_kind[off] == SPLASH_BLOCK_PARTIAL;
-        if (a.mask_desc && it.mask_head(it.g) != cur_mh) {
-          cur_mh = it.mask_head(it.g);
+        const int off = off_next, qblk = qblk_next;
+        const bool partial = kind_next == SPLASH_BLOCK_PARTIAL;
+        const bool seg_compare = has_seg && !it.uniform();
+        const int mh = it.mask_head(it.g);
+        it.next();
+        if (it.valid()) {  // the next step's entries are on their way while this one is worked on
+          off_next = it.off();
+          qblk_next = a.block_list[off_next];
+          kind_next = a.block_kind[off_next];
+        }
+        if (a.mask_desc && mh != cur_mh) {
+          cur_mh = mh;
           band_lo = a.mask_desc[cur_mh * 4 + 0];
           band_hi = a.mask_desc[cur_mh * 4 + 1];
           const int chunk = a.mask_desc[cur_mh * 4 + 2];
@@ -483,10 +495,15 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         const int q0 = qblk * 128 + col0;  // sequence position of this thread's first column
         // Visibility of this thread's 64 columns (bit i of word c: column c * 32 + i).
         uint32_t vis[2] = {0xffffffffu, 0xffffffffu};
-        const bool seg_compare = has_seg && !it.uniform();
         const bool plain_step = !partial && !seg_compare && !cap_on;
         if (!plain_step) {
-          if (partial) {
+          if (partial && a.partial_blocks) {
+            // Transposed block, one bit per element: 16 bytes per kv row, bit = q column.
+            const uint2 bits = __ldg(reinterpret_cast<const uint2*>(
+                a.partial_blocks + static_cast<size_t>(a.mask_block[off]) * (kRows * 16) + row * 16 + w * 8));
+            vis[0] = bits.x;
+            vis[1] = bits.y;
+          } else if (partial) {
             // Column i of word c is visible iff band_lo <= d0 - i <= band_hi: a run of bits.
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
@@ -533,41 +550,45 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           auto body = [&](auto cap_c, auto mask_c) {
             constexpr bool kCap = decltype(cap_c)::value, kMask = decltype(mask_c)::value;
             constexpr bool kNeedLse = kCap || !L::kFold;
+const float2 scale2 = make_float2(kCap ? cap * kLog2e : kLog2e, kCap ? cap * kLog2e : kLog2e);
 #pragma unroll
             for (int g = 0; g < 16; ++g) {
-              float nl[4] = {0.f, 0.f, 0.f, 0.f};
+              float2 nl[2];
               if constexpr (kNeedLse) {
                 const uint4 lw = lds128(vec + g * 16);
-                const uint32_t lraw[4] = {lw.x, lw.y, lw.z, lw.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float lse_e = __uint_as_float(lraw[e]);
-                  nl[e] = lse_e * -kLog2e;
-                  if constexpr (kMask) {
-                    if (lse_e == a.mask_value) nl[e] = -INFINITY;
-                  }
-                }
-              }
-              float pv[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int i = g * 4 + e;
-                float sval = pf[i], keep = 1.f;
-                if constexpr (kCap) {
-                  const float th = tanh_approx(sval * inv_cap);
-                  sval = cap * th;
-                  keep = fmaf(-th, th, 1.f);
-                }
-                float x = kNeedLse ? fmaf(sval, kLog2e, nl[e]) : sval * kLog2e;
+                const float2 l01 = make_float2(__uint_as_float(lw.x), __uint_as_float(lw.y));
+                const float2 l23 = make_float2(__uint_as_float(lw.z), __uint_as_float(lw.w));
+                nl[0] = mul2(l01, make_float2(-kLog2e, -kLog2e));
+                nl[1] = mul2(l23, make_float2(-kLog2e, -kLog2e));
                 if constexpr (kMask) {
-                  if (!((vis[i >> 5] >> (i & 31)) & 1u)) x = -INFINITY;
+                  if (l01.x == a.mask_value) nl[0].x = -INFINITY;
+                  if (l01.y == a.mask_value) nl[0].y = -INFINITY;
+                  if (l23.x == a.mask_value) nl[1].x = -INFINITY;
+                  if (l23.y == a.mask_value) nl[1].y = -INFINITY;
                 }
-                const float p = ex2_approx(x);
-                pv[e] = p;
-                pf[i] = kCap ? p * keep : p;
               }
-              ppk[g * 2] = pack2<BF16>(pv[0], pv[1]);
-              ppk[g * 2 + 1] = pack2<BF16>(pv[2], pv[3]);
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const int i = g * 4 + e * 2;
+                float2 sval = make_float2(pf[i], pf[i + 1]), keep = make_float2(1.f, 1.f);
+                if constexpr (kCap) {
+                  // cap * tanh(s / cap), with cap folded into the scale of the exponent.
+                  sval = mul2(sval, make_float2(inv_cap, inv_cap));
+                  sval.x = tanh_approx(sval.x);
+                  sval.y = tanh_approx(sval.y);
+                  keep = fma2(make_float2(-sval.x, -sval.y), sval, make_float2(1.f, 1.f));
+                }
+                float2 x = kNeedLse ? fma2(sval, scale2, nl[e]) : mul2(sval, scale2);
+                if constexpr (kMask) {
+                  if (!((vis[i >> 5] >> (i & 31)) & 1u)) x.x = -INFINITY;
+                  if (!((vis[i >> 5] >> ((i + 1) & 31)) & 1u)) x.y = -INFINITY;
+                }
+                const float2 p = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+                ppk[g * 2 + e] = pack2<BF16>(p.x, p.y);
+                const float2 f = kCap ? mul2(p, keep) : p;
+                pf[i] = f.x;
+                pf[i + 1] = f.y;
+              }
             }
           };
           using T = std::true_type;
@@ -595,27 +616,21 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           tmem_ld32(tmem_row + L::kColDp + col0 + c * 32, dpraw);
           tmem_wait_ld();
           uint32_t dspk[16];
-          if constexpr (L::kFold) {
-            // dP^T arrives with delta already subtracted.
+          const uint32_t vec = delta_u32 + slot * L::kVecBytes + (col0 + c * 32) * 4;
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              const int i = c * 32 + g * 4;
-              dspk[g * 2] = pack2<BF16>(pf[i + 0] * __uint_as_float(dpraw[g * 4 + 0]),
-                                        pf[i + 1] * __uint_as_float(dpraw[g * 4 + 1]));
-              dspk[g * 2 + 1] = pack2<BF16>(pf[i + 2] * __uint_as_float(dpraw[g * 4 + 2]),
-                                            pf[i + 3] * __uint_as_float(dpraw[g * 4 + 3]));
-            }
-          } else {
-            const uint32_t vec = delta_u32 + slot * L::kVecBytes + (col0 + c * 32) * 4;
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {
+          for (int g = 0; g < 8; ++g) {
+            const int i = c * 32 + g * 4;
+            float2 d01 = make_float2(__uint_as_float(dpraw[g * 4 + 0]), __uint_as_float(dpraw[g * 4 + 1]));
+            float2 d23 = make_float2(__uint_as_float(dpraw[g * 4 + 2]), __uint_as_float(dpraw[g * 4 + 3]));
+            if constexpr (!L::kFold) {  // where delta is folded in, dP^T arrives with it subtracted
               const uint4 dw = lds128(vec + g * 16);
-              const int i = c * 32 + g * 4;
-              dspk[g * 2] = pack2<BF16>(pf[i + 0] * (__uint_as_float(dpraw[g * 4 + 0]) - __uint_as_float(dw.x)),
-                                        pf[i + 1] * (__uint_as_float(dpraw[g * 4 + 1]) - __uint_as_float(dw.y)));
-              dspk[g * 2 + 1] = pack2<BF16>(pf[i + 2] * (__uint_as_float(dpraw[g * 4 + 2]) - __uint_as_float(dw.z)),
-                                            pf[i + 3] * (__uint_as_float(dpraw[g * 4 + 3]) - __uint_as_float(dw.w)));
+              d01 = sub2(d01, make_float2(__uint_as_float(dw.x), __uint_as_float(dw.y)));
+              d23 = sub2(d23, make_float2(__uint_as_float(dw.z), __uint_as_float(dw.w)));
             }
+            d01 = mul2(d01, make_float2(pf[i], pf[i + 1]));
+            d23 = mul2(d23, make_float2(pf[i + 2], pf[i + 3]));
+            dspk[g * 2] = pack2<BF16>(d01.x, d01.y);
+            dspk[g * 2 + 1] = pack2<BF16>(d23.x, d23.y);
           }
           tmem_st16(tmem_row + L::kColDp + col0 + c * 16, dspk);
           // dS^T staged as [kv row][q], two boxes of 64 q columns, 128-byte swizzle.

@@ -15,7 +15,7 @@ int launch_fwd(const SplashParams& p, cudaStream_t stream);
 
 namespace splash {
 
-template <int D, int DV, bool FUSED>
+template <int D, int DV>
 int launch_bwd_col(const SplashParams& p, cudaStream_t stream);
 
 template <int D, int DV, int BC>
@@ -24,8 +24,7 @@ int launch_bwd_row(const SplashParams& p, cudaStream_t stream);
 template <int D, int DV, int BC>
 size_t bwd_row_smem(const SplashParams& p);
 
-// Fused backward with 128 q rows per step (head_dim 128, no streamed mask blocks).
-bool bwd_wide_supported(const SplashParams& p);
+// Fused backward, 128 q rows per step (head_dim == head_dim_v, 64 or 128).
 int launch_bwd_wide(const SplashParams& p, cudaStream_t stream);
 
 // delta = rowsum(dO * O); dq = cast(transpose(dq_acc)).
