@@ -77,9 +77,9 @@ typedef struct SplashParams {
   void* dq;         /* backward: like q                                         */
   void* dk;         /* backward: like k                                         */
   void* dv;         /* backward: like v                                         */
-  float* dq_acc;    /* fused backward scratch: f32, transposed -- [batch, heads, head_dim, q_len],
-                     * i.e. [batch * heads * head_dim, q_len] row-major; size from
-                     * splash_bwd_fused_workspace_bytes()                         */
+  float* dq_acc;    /* fused backward scratch, 16-byte aligned: f32 accumulator, [batch, heads,
+                     * head_dim, q_len] at head_dim 128 and [batch, heads, q_len, head_dim] at
+                     * 64; size from splash_bwd_fused_workspace_bytes()           */
   int32_t* status;  /* 4 x int32, see above                                     */
   /* ---- static configuration ---------------------------------------------- */
   int32_t batch, heads, kv_heads, q_len, kv_len, head_dim, head_dim_v;

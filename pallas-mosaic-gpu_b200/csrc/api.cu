@@ -161,7 +161,7 @@ extern "C" int splash_bwd_fused(const SplashParams* p, void* stream) {
     SPLASH_CUDA_CHECK(cudaMemsetAsync(p->dq_acc, 0, static_cast<size_t>(dq_acc_bytes(p)), st));
   }
   if (int rc = launch_bwd_wide(*p, st)) return rc;
-  return launch_dq_transpose_cast(p->dq_acc, p->dq, static_cast<long long>(p->batch) * p->heads, p->head_dim, p->q_len,
+  return launch_dq_cast(p->dq_acc, p->dq, static_cast<long long>(p->batch) * p->heads, p->head_dim, p->q_len,
                                   p->dtype, st);
 }
 

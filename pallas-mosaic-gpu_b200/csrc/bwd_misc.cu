@@ -1,13 +1,15 @@
 // Small memory-bound passes around the backward kernels:
 //   delta = rowsum(dO * O) in f32 (what the reference leaves to XLA,
 //           splash_attention_mgpu/splash_attention.py:289-290);
-//   dq    = cast(transpose(dq_acc)): the fused backward accumulates dQ^T in f32 as
-//           [batch*heads, head_dim, q_len] (reference backward_fused.py:506-511).
+//   dq    = cast(dq_acc): the fused backward accumulates dQ^T in f32 as [batch*heads, head_dim,
+//           q_len] at head_dim 128 (transposed on the way; reference backward_fused.py:506-511),
+//           dQ as [batch*heads, q_len, head_dim] at head_dim 64.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include "dispatch.h"
 #include "host_common.cuh"
+#include "ptx.cuh"
 
 namespace splash {
 
@@ -204,10 +206,29 @@ int launch_seg_ranges(const SplashParams& p, cudaStream_t stream) {
   return SPLASH_OK;
 }
 
-int launch_dq_transpose_cast(const float* acc, void* dq, long long batch_heads, int head_dim, int q_len, int dtype,
-                             cudaStream_t stream) {
+template <bool BF16>
+__global__ void __launch_bounds__(256) dq_cast_kernel(const float4* __restrict__ acc, uint4* __restrict__ dq, long long n8) {
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= n8) return;
+  const float4 a = acc[2 * i], b = acc[2 * i + 1];
+  dq[i] = make_uint4(pack2<BF16>(a.x, a.y), pack2<BF16>(a.z, a.w), pack2<BF16>(b.x, b.y), pack2<BF16>(b.z, b.w));
+}
+
+// The accumulator is [bh, q, d] at head_dim 64, [bh, d, q] at head_dim 128 (bwd_wide_kernel.cuh).
+int launch_dq_cast(const float* acc, void* dq, long long batch_heads, int head_dim, int q_len, int dtype,
+                   cudaStream_t stream) {
   if (!acc || !dq || head_dim % 64 || q_len % 64) return fail(SPLASH_INVALID_ARGUMENT, "bad dq cast arguments");
   if (batch_heads * (q_len / 64) >= (1ll << 31)) return fail(SPLASH_INVALID_ARGUMENT, "batch * heads * q_len too large");
+  if (head_dim == 64) {
+    const long long n8 = batch_heads * q_len * 8;  // 16-byte pieces of dq
+    const unsigned grid = static_cast<unsigned>((n8 + 255) / 256);
+    if (dtype == SPLASH_DTYPE_BF16)
+      dq_cast_kernel<true><<<grid, 256, 0, stream>>>(reinterpret_cast<const float4*>(acc), static_cast<uint4*>(dq), n8);
+    else
+      dq_cast_kernel<false><<<grid, 256, 0, stream>>>(reinterpret_cast<const float4*>(acc), static_cast<uint4*>(dq), n8);
+    SPLASH_CUDA_CHECK(cudaGetLastError());
+    return SPLASH_OK;
+  }
   dim3 grid(static_cast<unsigned>(batch_heads * (q_len / 64)), head_dim / 64, 1);
   if (dtype == SPLASH_DTYPE_BF16)
     dq_transpose_cast_kernel<true><<<grid, 256, 0, stream>>>(acc, static_cast<uint16_t*>(dq), head_dim, q_len);

@@ -20,9 +20,10 @@ static int launch_bwd_wide_typed(const SplashParams& p, cudaStream_t stream) {
   if ((rc = make_tmap_2d(&tm_v, p.v, dt, 2, kv_rows, D, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   if ((rc = make_tmap_2d(&tm_dk, p.dk, dt, 2, kv_rows, D, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   if ((rc = make_tmap_2d(&tm_dv, p.dv, dt, 2, kv_rows, D, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
-  // f32 accumulator viewed as [batch * heads * head_dim, q_len]; tiles of 32 rows x 32 q columns.
-  const uint64_t acc_rows = static_cast<uint64_t>(p.batch) * p.heads * D;
-  if ((rc = make_tmap_2d(&tm_dqacc, p.dq_acc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, acc_rows, p.q_len, 32, 32,
+  // f32 accumulator, tiles of 32 x 32: [batch * heads * head_dim, q_len], at head_dim 64
+  // [batch * heads * q_len, head_dim].
+  const uint64_t acc_rows = L::kRoomy ? q_rows : static_cast<uint64_t>(p.batch) * p.heads * D;
+  if ((rc = make_tmap_2d(&tm_dqacc, p.dq_acc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, acc_rows, L::kRoomy ? D : p.q_len, 32, 32,
                          CU_TENSOR_MAP_SWIZZLE_128B)))
     return rc;
   if (reinterpret_cast<uintptr_t>(p.partial_blocks) & 15)

@@ -23,7 +23,7 @@
 //   dQ^T = K^T dS^T     smem x smem -> R2, drained by a writer warpgroup that
 //                       reduce-adds it into the f32 accumulator [batch*heads*128, q_len]
 //
-// Tensor memory holds R1, R2, dK and dV (4 x 128 = 512 columns), so the scores are not
+// At head_dim 128 tensor memory holds R1, R2, dK and dV (4 x 128 = 512 columns), so the scores are not
 // double-buffered; the overlap comes from the issue order instead:
 //   dP^T(t)  dV(t)  S^T(t+1)  dK(t)  dQ^T(t)  [writer drains R2]  dP^T(t+1) ...
 // Phase B of step t runs under dV(t) and S^T(t+1); phase A of step t+1 runs under dK(t),
@@ -32,6 +32,14 @@
 // (it lives from dP^T(t) to dV(t), which are adjacent) and is refilled under S^T(t+1),
 // dK(t) and dQ^T(t).  The writer stages f32 dQ^T tiles in 32 KB of its own, so it only
 // has to keep up with the step rate.
+//
+// At head_dim 64 dK and dV take 64 columns each, and the other 128 hold P^T and dQ:
+//   S^T(t+1)  dV(t)  dK(t)  dP^T(t+1)  dQ(t) ...
+// S^T(t+1) is issued as soon as S^T(t) stands in registers, dP^T(t+1) right behind dK(t), and nobody
+// waits for the drain.  dQ is formed as [q, d] with M = 128 q rows; as [d, q] its 64 rows had to be
+// doubled to fill the 128.  Measured (causal, 64 heads, seq 8192, f16): backward call 1672 -> 1539 us;
+// a step takes 2450-2550 cycles, of which the tensor core is busy 1370, and is paced by the
+// elementwise warps that share a scheduler with the issuing warp.
 //
 // Behaviour follows the reference kernel (splash_attention_mgpu/backward_fused.py:64-512);
 // the code shares nothing with it.
@@ -55,7 +63,7 @@ namespace splash {
 enum WideSite : int {
   kWSiteQEmpty = 61, kWSiteDoEmpty, kWSiteMmaKV, kWSiteMmaQ, kWSiteMmaDo, kWSiteMmaP, kWSiteMmaDs, kWSiteMmaDqFree,
   kWSiteEwQ, kWSiteEwS, kWSiteEwDp, kWSiteEwStage, kWSiteEwDone, kWSiteEwEpi,
-  kWSiteWrReady,
+  kWSiteWrReady, kWSiteMmaSFree,
 };
 
 template <int D_>
@@ -66,16 +74,20 @@ struct WideLayout {
   static constexpr int BC = 128;     // q rows per step
   static constexpr int kBox = kRows * 128;        // one 64-element-wide box of a 128-row tile: 16 KB
   static constexpr int kTile = kRows * D * 2;     // a K, V, Q or dO tile
-  // At head_dim 64 the dQ^T product keeps M = 128: its A operand's second 64 rows are a second
-  // copy of the K tile, so the upper half of the result repeats the lower half and is not stored.
-  static constexpr int kKDupBytes = D == 64 ? kBox : 0;
   static constexpr int kDsBytes = kRows * BC * 2;  // dS^T as an MMA operand
+  // Head_dim 64 leaves room in both memories (kRoomy): P^T and dQ have tensor-memory columns of their
+  // own, dO and the staged dS^T a second buffer each, which takes P^T -> dV -> S^T(t+1) and
+  // dQ -> drain -> dP^T(t+1) off the critical path of a step.  dQ is then formed as [q, d] (64
+  // columns) instead of [d, q].
+  static constexpr bool kRoomy = D == 64;
   static constexpr int kSlots = 2;
+  static constexpr int kDoSlots = kRoomy ? 2 : 1;
+  static constexpr int kDsBufs = kRoomy ? 2 : 1;
   static constexpr int kVecBytes = BC * 4;
   // Shared memory map (bytes from the 1024-aligned base).
-  static constexpr int kOffK = 0, kOffV = kTile + kKDupBytes, kOffQ = kOffV + kTile, kOffDo = kOffQ + kSlots * kTile;
-  static constexpr int kOffDs = kOffDo + kTile;
-  static constexpr int kOffDqStage = kOffDs + kDsBytes;  // per writer warp: kDqBufs f32 tiles of [32 d, 32 q]
+  static constexpr int kOffK = 0, kOffV = kTile, kOffQ = kOffV + kTile, kOffDo = kOffQ + kSlots * kTile;
+  static constexpr int kOffDs = kOffDo + kDoSlots * kTile;
+  static constexpr int kOffDqStage = kOffDs + kDsBufs * kDsBytes;  // per writer warp: kDqBufs f32 tiles of [32 d, 32 q]
   static constexpr int kDqBufs = 2;
   static constexpr int kDqBoxBytes = 32 * 32 * 4;
   static constexpr int kOffLse = kOffDqStage + 4 * kDqBufs * kDqBoxBytes, kOffDelta = kOffLse + kSlots * kVecBytes;
@@ -94,8 +106,11 @@ struct WideLayout {
   static constexpr int kListSteps = 256;  // capacity of the list of block steps that survive segment skipping
   static constexpr int kOffList = kOffBars + kBarBytes;
   static constexpr int kSmemBytes = kOffList + kListSteps * 2;
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory per CTA");
   // Tensor memory columns.
   static constexpr int kColS = 0, kColDp = 128, kColDk = 256, kColDv = 256 + D;
+  static constexpr int kColP = kRoomy ? 384 : kColS, kColDq = kRoomy ? 448 : kColDp;
+  static constexpr int kPHalf = kRoomy ? 32 : 64;  // columns from the packed P^T of one warpgroup to the other's
   static constexpr int kTmemCols = 512;
   static constexpr int kEwThreads = 256;
   static constexpr int kThreads = 512;  // 2 elementwise warpgroups, writer warpgroup, producer warpgroup
@@ -103,10 +118,20 @@ struct WideLayout {
   static constexpr int kEwRegs = 160, kWriterRegs = 152, kProducerRegs = 40;
 };
 
+// Position in a ring of N slots, and the parity of its barriers there.
+template <int N>
+struct Ring {
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++slot == N) { slot = 0; phase ^= 1; }
+  }
+};
+
 struct WideBarriers {
   uint64_t kv_full;
-  uint64_t q_full[2], q_empty[2], do_full, do_empty;
-  uint64_t s_ready, dp_ready, p_ready, ds_ready;
+  uint64_t q_full[2], q_empty[2], do_full[2], do_empty[2];
+  uint64_t s_ready, s_free, dp_ready, p_ready, ds_ready;
   uint64_t dq_ready, dq_free;
   uint64_t acc_done, epi[2];
   uint32_t tmem_base;
@@ -190,7 +215,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       const uint32_t off = 8u * i;
       uint32_t count = 1;
       if (off >= offsetof(WideBarriers, q_empty) && off < offsetof(WideBarriers, do_full)) count = 1 + kEwWarps;  // dK + vector readers
-      if (off == offsetof(WideBarriers, p_ready) || off == offsetof(WideBarriers, ds_ready)) count = L::kEwThreads;
+      if (off == offsetof(WideBarriers, s_free) || off == offsetof(WideBarriers, p_ready) || off == offsetof(WideBarriers, ds_ready)) count = L::kEwThreads;
       if (off == offsetof(WideBarriers, dq_free) || off >= offsetof(WideBarriers, epi)) count = 128;
       mbar_init(bars_u32 + off, count);
     }
@@ -257,18 +282,18 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         prefetch_tensormap(&tm_q);
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
-        mbar_arrive_expect_tx(SPLASH_WBAR(kv_full, 0), 2 * L::kTile + L::kKDupBytes);
+        mbar_arrive_expect_tx(SPLASH_WBAR(kv_full, 0), 2 * L::kTile);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) tma_load_2d(k_u32 + c * L::kBox, &tm_k, c * 64, kv_row0, SPLASH_WBAR(kv_full, 0));
-        if constexpr (L::kKDupBytes > 0) tma_load_2d(k_u32 + L::kTile, &tm_k, 0, kv_row0, SPLASH_WBAR(kv_full, 0));
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) tma_load_2d(v_u32 + c * L::kBox, &tm_v, c * 64, kv_row0, SPLASH_WBAR(kv_full, 0));
       }
-      for (int t = 0; it.valid(); it.next(), ++t) {
-        const int slot = t & 1;
+      Ring<L::kSlots> q;
+      for (int t = 0; it.valid(); it.next(), ++t, q.next()) {
+        const int slot = q.slot;
         const int qblk = a.block_list[it.off()];
         const int q_row = (b * a.heads + it.head()) * a.q_len + qblk * 128;
-        if (t >= 2 && !warp_wait(SPLASH_WBAR(q_empty, slot), ((t >> 1) & 1) ^ 1, ctx, kWSiteQEmpty, t)) break;
+        if (t >= L::kSlots && !warp_wait(SPLASH_WBAR(q_empty, slot), q.phase ^ 1, ctx, kWSiteQEmpty, t)) break;
         if (elect_one()) {
           const uint32_t bar = SPLASH_WBAR(q_full, slot);
           mbar_arrive_expect_tx(bar, L::kTile + (L::kFold ? 2 * L::kAuxTile + L::kVecBytes : 2 * L::kVecBytes));
@@ -287,15 +312,18 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     } else if (warp == kProducerWarp0 + 2 && total > 0) {
       // ------------------------------------ dO ring ------------------------------------
       if (elect_one()) prefetch_tensormap(&tm_do);
-      for (int t = 0; it.valid(); it.next(), ++t) {
+      Ring<L::kDoSlots> d;
+      for (int t = 0; it.valid(); it.next(), ++t, d.next()) {
+        const int slot = d.slot;
         const int qblk = a.block_list[it.off()];
         const int q_row = (b * a.heads + it.head()) * a.q_len + qblk * 128;
-        if (t >= 1 && !warp_wait(SPLASH_WBAR(do_empty, 0), (t & 1) ^ 1, ctx, kWSiteDoEmpty, t)) break;
+        if (t >= L::kDoSlots && !warp_wait(SPLASH_WBAR(do_empty, slot), d.phase ^ 1, ctx, kWSiteDoEmpty, t)) break;
         if (elect_one()) {
-          const uint32_t bar = SPLASH_WBAR(do_full, 0);
+          const uint32_t bar = SPLASH_WBAR(do_full, slot);
           mbar_arrive_expect_tx(bar, L::kTile);
 #pragma unroll
-          for (int c = 0; c < D / 64; ++c) tma_load_2d(do_u32 + c * L::kBox, &tm_do, c * 64, q_row, bar);
+          for (int c = 0; c < D / 64; ++c)
+            tma_load_2d(do_u32 + slot * L::kTile + c * L::kBox, &tm_do, c * 64, q_row, bar);
         }
       }
     } else if (warp == kProducerWarp0 + 1 && total > 0) {
@@ -303,7 +331,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       // All lanes run the loop; one elected lane issues each instruction.
       constexpr uint32_t kIdescScore = make_idesc(BF16, 128, 128, false, false);  // K Q^T, V dO^T
       constexpr uint32_t kIdescAcc = make_idesc(BF16, 128, D, false, true);        // P^T dO, dS^T Q
-      constexpr uint32_t kIdescDq = make_idesc(BF16, 128, 128, true, true);        // K^T dS^T
+      constexpr uint32_t kIdescDq = make_idesc(BF16, 128, D, true, true);         // dS K, K^T dS^T
       // K-major tiles: 64-element boxes side by side, 32 bytes per 16-element slice.
       auto issue_scores = [&](uint32_t d_col, uint32_t a_tile, uint32_t b_tile) {
         const uint32_t a_lo = desc_lo(a_tile, 16), b_lo = desc_lo(b_tile, 16);
@@ -322,19 +350,21 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       // A = packed 16-bit values the elementwise warps left in tensor memory: q columns
       // 0-63 packed into columns 0-31 of the region, q columns 64-127 into columns 64-95
       // (each warpgroup packs into its own half).  B = a [128 q, 128 d] tile read MN-major.
-      auto issue_acc = [&](uint32_t d_col, uint32_t a_col, uint32_t b_tile, bool first) {
+      auto issue_acc = [&](uint32_t d_col, uint32_t a_col, uint32_t a_half, uint32_t b_tile, bool first) {
         const uint32_t b_lo = desc_lo(b_tile, L::kBox);
 #pragma unroll
         for (int kk = 0; kk < 128 / 16; ++kk)
-          umma_ts2_w(tmem + d_col, tmem + a_col + (kk >> 2) * 64 + (kk & 3) * 8, b_lo + ((kk * 2048) >> 4), kDescHi,
+          umma_ts2_w(tmem + d_col, tmem + a_col + (kk >> 2) * a_half + (kk & 3) * 8, b_lo + ((kk * 2048) >> 4), kDescHi,
                      kIdescAcc, (!first || kk > 0) ? 1u : 0u);
       };
-      // dQ^T[d, q] = sum_kv K[kv, d] dS^T[kv, q]: both operands read MN-major.
-      auto issue_dq = [&]() {
-        const uint32_t k_lo = desc_lo(k_u32, L::kBox), ds_lo = desc_lo(ds_u32, L::kBox);
+      // dQ^T[d, q] = sum_kv K[kv, d] dS^T[kv, q], or (kRoomy) dQ[q, d] with the operands exchanged;
+      // both are read MN-major.
+      auto issue_dq = [&](int buf) {
+        const uint32_t k_lo = desc_lo(k_u32, L::kBox), ds_lo = desc_lo(ds_u32 + buf * L::kDsBytes, L::kBox);
+        const uint32_t a_lo = L::kRoomy ? ds_lo : k_lo, b_lo = L::kRoomy ? k_lo : ds_lo;
 #pragma unroll
         for (int kk = 0; kk < kRows / 16; ++kk)
-          umma_ss2_w(tmem + L::kColDp, k_lo + ((kk * 2048) >> 4), kDescHi, ds_lo + ((kk * 2048) >> 4), kDescHi, kIdescDq,
+          umma_ss2_w(tmem + L::kColDq, a_lo + ((kk * 2048) >> 4), kDescHi, b_lo + ((kk * 2048) >> 4), kDescHi, kIdescDq,
                      kk > 0);
       };
       bool ok = warp_wait(SPLASH_WBAR(kv_full, 0), 0, ctx, kWSiteMmaKV, 0) &&
@@ -348,45 +378,71 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       }
       if (ok) {
         tc_fence_after();
-        issue_scores(L::kColDp, v_u32, do_u32);
+        issue_scores(L::kColDp, v_u32, do_u32);  // dO slot 0
         if constexpr (L::kFold) issue_fold(L::kColDp, aux_u32 + L::kAuxTile);
         umma_commit_w(SPLASH_WBAR(dp_ready, 0));
-        for (int t = 0; t < total; ++t) {
-          const int slot = t & 1, nslot = slot ^ 1;
+        Ring<L::kSlots> q, nq;            // Q slot of this step and of the next
+        Ring<L::kDoSlots> d, nd;          // dO likewise
+        nq.next();
+        nd.next();
+        for (int t = 0; t < total; ++t, q = nq, nq.next(), d = nd, nd.next()) {
           const uint32_t par = t & 1;
+          const bool more = t + 1 < total;
+          auto next_s = [&]() -> bool {                                        // S^T(t+1)
+            if (!warp_wait(SPLASH_WBAR(q_full, nq.slot), nq.phase, ctx, kWSiteMmaQ, t + 1)) return false;
+            SPLASH_TRACE_MARK(0, t, 2);
+            if constexpr (L::kRoomy) {
+              if (!warp_wait(SPLASH_WBAR(s_free, 0), par, ctx, kWSiteMmaSFree, t)) return false;
+            }
+            tc_fence_after();
+            issue_scores(L::kColS, k_u32, q_u32 + nq.slot * L::kTile);
+            if (fold_lse) issue_fold(L::kColS, aux_u32 + nq.slot * 2 * L::kAuxTile);
+            umma_commit_w(SPLASH_WBAR(s_ready, 0));
+            return true;
+          };
+          auto next_dp = [&]() -> bool {                                       // dP^T(t+1) over dS^T(t)
+            if (!warp_wait(SPLASH_WBAR(do_full, nd.slot), nd.phase, ctx, kWSiteMmaDo, t + 1)) return false;
+            tc_fence_after();
+            issue_scores(L::kColDp, v_u32, do_u32 + nd.slot * L::kTile);
+            if constexpr (L::kFold) issue_fold(L::kColDp, aux_u32 + nq.slot * 2 * L::kAuxTile + L::kAuxTile);
+            umma_commit_w(SPLASH_WBAR(dp_ready, 0));
+            return true;
+          };
           SPLASH_TRACE_MARK(0, t, 0);
+          if constexpr (L::kRoomy) {
+            if (more && !next_s()) break;                                      // the row of S^T(t) is in registers
+          }
           if (!warp_wait(SPLASH_WBAR(p_ready, 0), par, ctx, kWSiteMmaP, t)) break;
           SPLASH_TRACE_MARK(0, t, 1);
           tc_fence_after();
-          issue_acc(L::kColDv, L::kColS, do_u32, t == 0);                      // dV += P^T dO
-          umma_commit_w(SPLASH_WBAR(do_empty, 0));
-          if (t + 1 < total) {
-            if (!warp_wait(SPLASH_WBAR(q_full, nslot), ((t + 1) >> 1) & 1, ctx, kWSiteMmaQ, t + 1)) break;
-            SPLASH_TRACE_MARK(0, t, 2);
-            tc_fence_after();
-            issue_scores(L::kColS, k_u32, q_u32 + nslot * L::kTile);         // S^T(t+1) over P^T(t)
-            if (fold_lse) issue_fold(L::kColS, aux_u32 + nslot * 2 * L::kAuxTile);
-            umma_commit_w(SPLASH_WBAR(s_ready, 0));
+          issue_acc(L::kColDv, L::kColP, L::kPHalf, do_u32 + d.slot * L::kTile, t == 0);  // dV += P^T dO
+          umma_commit_w(SPLASH_WBAR(do_empty, d.slot));
+          if constexpr (!L::kRoomy) {
+            if (more && !next_s()) break;                                      // over P^T(t)
           }
           SPLASH_TRACE_MARK(0, t, 3);
           if (!warp_wait(SPLASH_WBAR(ds_ready, 0), par, ctx, kWSiteMmaDs, t)) break;
           SPLASH_TRACE_MARK(0, t, 4);
           tc_fence_after();
-          issue_acc(L::kColDk, L::kColDp, q_u32 + slot * L::kTile, t == 0);   // dK += dS^T Q
-          umma_commit_w(SPLASH_WBAR(q_empty, slot));
-          issue_dq();                                                          // dQ^T(t) over dS^T(t)
-          umma_commit_w(SPLASH_WBAR(dq_ready, 0));
-          SPLASH_TRACE_MARK(0, t, 5);
-          if (t + 1 < total && !warp_wait(SPLASH_WBAR(do_full, 0), par ^ 1, ctx, kWSiteMmaDo, t + 1)) break;
-          SPLASH_TRACE_MARK(0, t, 6);
-          // The writer must have taken dQ^T(t) out of R2 (every phase of dq_free is observed).
-          if (!warp_wait(SPLASH_WBAR(dq_free, 0), par, ctx, kWSiteMmaDqFree, t)) break;
-          SPLASH_TRACE_MARK(0, t, 7);
-          if (t + 1 < total) {
+          issue_acc(L::kColDk, L::kColDp, 64, q_u32 + q.slot * L::kTile, t == 0);         // dK += dS^T Q
+          umma_commit_w(SPLASH_WBAR(q_empty, q.slot));
+          if constexpr (L::kRoomy) {
+            if (more && !next_dp()) break;
+            SPLASH_TRACE_MARK(0, t, 5);
+            // The writer must have taken dQ(t-1) out of its columns.
+            if (t > 0 && !warp_wait(SPLASH_WBAR(dq_free, 0), par ^ 1, ctx, kWSiteMmaDqFree, t)) break;
+            SPLASH_TRACE_MARK(0, t, 6);
             tc_fence_after();
-            issue_scores(L::kColDp, v_u32, do_u32);                            // dP^T(t+1)
-            if constexpr (L::kFold) issue_fold(L::kColDp, aux_u32 + nslot * 2 * L::kAuxTile + L::kAuxTile);
-            umma_commit_w(SPLASH_WBAR(dp_ready, 0));
+            issue_dq(t & 1);
+            umma_commit_w(SPLASH_WBAR(dq_ready, 0));
+          } else {
+            issue_dq(0);                                                       // dQ^T(t) over dS^T(t)
+            umma_commit_w(SPLASH_WBAR(dq_ready, 0));
+            SPLASH_TRACE_MARK(0, t, 5);
+            // The writer must have taken dQ^T(t) out of R2 (every phase of dq_free is observed).
+            if (!warp_wait(SPLASH_WBAR(dq_free, 0), par, ctx, kWSiteMmaDqFree, t)) break;
+            SPLASH_TRACE_MARK(0, t, 7);
+            if (more && !next_dp()) break;
           }
         }
         umma_commit_w(SPLASH_WBAR(acc_done, 0));
@@ -398,7 +454,8 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     // Each warp drains its own 32 head-dim rows (its quarter of the TMEM lanes) through
     // staging tiles of its own, so the writer warps never wait for one another.
     const int wq = warp & 3;
-    const uint32_t dq_tmem = tmem + (static_cast<uint32_t>(wq * 32) << 16) + L::kColDp;
+    constexpr int kTiles = D / 32;  // [32, 32] tiles per warp and step
+    const uint32_t dq_tmem = tmem + (static_cast<uint32_t>(wq * 32) << 16) + L::kColDq;
     const uint32_t my_stage = dqs_u32 + wq * (L::kDqBufs * L::kDqBoxBytes);
     int t = 0;
     for (; it.valid(); it.next(), ++t) {
@@ -407,22 +464,20 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       if (!warp_wait(SPLASH_WBAR(dq_ready, 0), t & 1, ctx, kWSiteWrReady, t)) break;
       SPLASH_TRACE_MARK(2, t, 1);
       tc_fence_after();
-      uint32_t acc[128];
-      const bool mine = wq * 32 < D;  // at head_dim 64 the upper two quarters repeat the lower ones
-      if (mine) {
+      uint32_t acc[kTiles * 32];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32(dq_tmem + c * 32, acc + c * 32);
-        tmem_wait_ld();
-      }
+      for (int c = 0; c < kTiles; ++c) tmem_ld32(dq_tmem + c * 32, acc + c * 32);
+      tmem_wait_ld();
       tc_fence_before();
       mbar_arrive(SPLASH_WBAR(dq_free, 0));
-      if (!mine) continue;
       SPLASH_TRACE_MARK(2, t, 2);
-      const int x = qblk * 128;
-      const int y = (b * a.heads + it.head()) * D + wq * 32;
-      // Four passes of 32 q columns: [32 d, 32 q] f32 tiles, 128-byte rows, 128-byte swizzle.
+      // dQ^T: the warp's 32 d rows, tiles of 32 q; dQ (kRoomy): its 32 q rows, tiles of 32 d.
+      const int x = L::kRoomy ? 0 : qblk * 128;
+      const int y = L::kRoomy ? (b * a.heads + it.head()) * a.q_len + qblk * 128 + wq * 32
+                              : (b * a.heads + it.head()) * D + wq * 32;
+      // f32 tiles of 32 rows of 128 bytes, 128-byte swizzle.
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < kTiles; ++j) {
         const uint32_t stage = my_stage + (j % L::kDqBufs) * L::kDqBoxBytes;
         // The reduction that last used this tile must have read it.
         if (lane == 0 && (t > 0 || j >= L::kDqBufs)) bulk_wait_group_read<L::kDqBufs - 1>();
@@ -465,10 +520,11 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       int cur_mh = -1;
       int band_lo = -(1 << 30), band_hi = (1 << 30);  // allowed range of kv_pos - q_pos for this kv row
 
+      Ring<L::kSlots> q;
       int off_next = it.off();
       int qblk_next = a.block_list[off_next], kind_next = a.block_kind[off_next];
-      for (int t = 0; t < total; ++t) {
-        const int slot = t & 1;
+      for (int t = 0; t < total; ++t, q.next()) {
+        const int slot = q.slot;
         const uint32_t par = t & 1;
         const int off = off_next, qblk = qblk_next;
         const bool partial = kind_next == SPLASH_BLOCK_PARTIAL;
@@ -527,7 +583,8 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         }
         SPLASH_TRACE_MARK(1, t, 0);
         SPLASH_TRACE_NS(1, t, 7);
-        if (!warp_wait(SPLASH_WBAR(q_full, slot), (t >> 1) & 1, ctx, kWSiteEwQ, t)) { alive = false; break; }
+        // (The vectors of the slot; without them to read the scores say enough.)
+        if ((!L::kFold || cap_on) && !warp_wait(SPLASH_WBAR(q_full, slot), q.phase, ctx, kWSiteEwQ, t)) { alive = false; break; }
         if (!warp_wait(SPLASH_WBAR(s_ready, 0), par, ctx, kWSiteEwS, t)) { alive = false; break; }
         SPLASH_TRACE_MARK(1, t, 1);
         tc_fence_after();
@@ -539,6 +596,10 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           tmem_ld32(tmem_row + L::kColS + col0, sraw);
           tmem_ld32(tmem_row + L::kColS + col0 + 32, sraw + 32);
           tmem_wait_ld();
+          if constexpr (L::kRoomy) {
+            tc_fence_before();
+            mbar_arrive(SPLASH_WBAR(s_free, 0));
+          }
           uint32_t ppk[32];
           const uint32_t vec = lse_u32 + slot * L::kVecBytes + col0 * 4;
           // One straight-line body per (soft-cap, masking) combination; the step picks one.
@@ -550,7 +611,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           auto body = [&](auto cap_c, auto mask_c) {
             constexpr bool kCap = decltype(cap_c)::value, kMask = decltype(mask_c)::value;
             constexpr bool kNeedLse = kCap || !L::kFold;
-const float2 scale2 = make_float2(kCap ? cap * kLog2e : kLog2e, kCap ? cap * kLog2e : kLog2e);
+            const float2 scale2 = make_float2(kCap ? cap * kLog2e : kLog2e, kCap ? cap * kLog2e : kLog2e);
 #pragma unroll
             for (int g = 0; g < 16; ++g) {
               float2 nl[2];
@@ -598,8 +659,14 @@ const float2 scale2 = make_float2(kCap ? cap * kLog2e : kLog2e, kCap ? cap * kLo
           else if (!cap_on) body(F{}, T{});
           else if (!masked) body(T{}, F{});
           else body(T{}, T{});
-          // Packed P^T goes over the first half of the columns this thread just read.
-          tmem_st32(tmem_row + L::kColS + col0, ppk);
+          if constexpr (L::kRoomy) {
+            // The tensor core runs its instructions in order: dP^T of this step comes after dV of the
+            // previous one, which read the P^T columns, and after the dQ that read the dS^T buffer.
+            if (!warp_wait(SPLASH_WBAR(dp_ready, 0), par, ctx, kWSiteEwDp, t)) { alive = false; break; }
+            tc_fence_after();
+          }
+          // Packed P^T; without columns of its own, over the first half of those this thread just read.
+          tmem_st32(tmem_row + L::kColP + w * L::kPHalf, ppk);
           tmem_wait_st();
           tc_fence_before();
           mbar_arrive(SPLASH_WBAR(p_ready, 0));
@@ -607,7 +674,7 @@ const float2 scale2 = make_float2(kCap ? cap * kLog2e : kLog2e, kCap ? cap * kLo
         SPLASH_TRACE_MARK(1, t, 2);
 
         // ---- phase B: dS^T from dP^T ---------------------------------------------------
-        if (!warp_wait(SPLASH_WBAR(dp_ready, 0), par, ctx, kWSiteEwDp, t)) { alive = false; break; }
+        if (!L::kRoomy && !warp_wait(SPLASH_WBAR(dp_ready, 0), par, ctx, kWSiteEwDp, t)) { alive = false; break; }
         SPLASH_TRACE_MARK(1, t, 3);
         tc_fence_after();
 #pragma unroll
@@ -636,7 +703,7 @@ const float2 scale2 = make_float2(kCap ? cap * kLog2e : kLog2e, kCap ? cap * kLo
           // dS^T staged as [kv row][q], two boxes of 64 q columns, 128-byte swizzle.
 #pragma unroll
           for (int g = 0; g < 4; ++g)
-            sts128(ds_u32 + w * L::kBox + swz128(row, c * 4 + g),
+            sts128(ds_u32 + (t % L::kDsBufs) * L::kDsBytes + w * L::kBox + swz128(row, c * 4 + g),
                    make_uint4(dspk[g * 4], dspk[g * 4 + 1], dspk[g * 4 + 2], dspk[g * 4 + 3]));
         }
         // The slot's vectors have been read.

@@ -27,12 +27,12 @@ size_t bwd_row_smem(const SplashParams& p);
 // Fused backward, 128 q rows per step (head_dim == head_dim_v, 64 or 128).
 int launch_bwd_wide(const SplashParams& p, cudaStream_t stream);
 
-// delta = rowsum(dO * O); dq = cast(transpose(dq_acc)).
+// delta = rowsum(dO * O); dq = cast(dq_acc), transposed where the accumulator is.
 // When `zero` is non-null the same pass also clears zero_floats_per_row floats per row of it.
 int launch_delta(const void* o, const void* d_out, float* delta, long long rows, int head_dim_v, int dtype,
                  cudaStream_t stream, float* zero = nullptr, int zero_floats_per_row = 0);
-int launch_dq_transpose_cast(const float* acc, void* dq, long long batch_heads, int head_dim, int q_len, int dtype,
-                             cudaStream_t stream);
+int launch_dq_cast(const float* acc, void* dq, long long batch_heads, int head_dim, int q_len, int dtype,
+                   cudaStream_t stream);
 // -lse and -delta of every q row as three 16-bit parts each (16 bytes per row and array): the
 // operands of the slice that the 128-row fused backward adds to its score products at head_dim 64.
 int launch_fold_operands(const float* lse, const float* delta, void* aux_lse, void* aux_delta, long long rows,
