@@ -153,12 +153,18 @@ extern "C" int splash_bwd_fused(const SplashParams* p, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (int rc = launch_seg_ranges(*p, st)) return rc;
   if (p->out) {
-    // One pass streams O and dO for delta and clears the accumulator on the way.
-    if (int rc = launch_delta(p->out, p->d_out, p->delta, static_cast<long long>(p->batch) * p->heads * p->q_len,
-                              p->head_dim_v, p->dtype, st, p->dq_acc, p->head_dim))
+    // One pass streams O and dO for delta, clears the accumulator on the way and (head_dim 64) writes
+    // the folded operands.
+    if (int rc = launch_delta(p->out, p->d_out, p->delta, q_row_count(*p), p->head_dim_v, p->dtype, st, p->dq_acc,
+                              p->head_dim, p->lse, fold_operand_lse(*p), fold_operand_delta(*p), p->mask_value))
       return rc;
   } else {
     SPLASH_CUDA_CHECK(cudaMemsetAsync(p->dq_acc, 0, static_cast<size_t>(dq_acc_bytes(p)), st));
+    if (fold_operand_lse(*p)) {
+      if (int rc = launch_fold_operands(p->lse, p->delta, fold_operand_lse(*p), fold_operand_delta(*p), q_row_count(*p),
+                                        p->mask_value, p->dtype, st))
+        return rc;
+    }
   }
   if (int rc = launch_bwd_wide(*p, st)) return rc;
   return launch_dq_cast(p->dq_acc, p->dq, static_cast<long long>(p->batch) * p->heads, p->head_dim, p->q_len,

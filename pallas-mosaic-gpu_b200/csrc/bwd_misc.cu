@@ -23,29 +23,66 @@ __device__ __forceinline__ float2 unpack2(uint32_t w) {
   }
 }
 
-// One warp per group of kRows rows; each lane handles 16-byte chunks (8 elements) and
-// keeps the loads of all its rows in flight together.  When `zero` is given, the warp
-// also clears `zero_vec_per_row` float4 per row of it: the fused backward gets its f32
-// dQ accumulator cleared by the pass that already streams O and dO.
+// Splits -x into three 16-bit floats whose sum is -x to f32 precision, as the eight 16-bit
+// values {hi, mid, lo, 0, 0, 0, 0, 0} per row that the 128-row fused backward (head_dim 64)
+// multiplies by {1, 1, 1, 0, ...} in one extra K = 16 slice of its score products.  Rows whose
+// lse is mask_value (they saw no key) get a large negative value instead, which makes their P zero.
+template <bool BF16>
+__device__ __forceinline__ uint4 split3_neg(float x, bool sentinel) {
+  float v = sentinel ? (BF16 ? -1.0e30f : -60000.f) : -x;
+  uint32_t h[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    if constexpr (BF16) {
+      const __nv_bfloat16 b = __float2bfloat16_rn(v);
+      h[i] = *reinterpret_cast<const uint16_t*>(&b);
+      v -= __bfloat162float(b);
+    } else {
+      const __half b = __float2half_rn(v);
+      h[i] = *reinterpret_cast<const uint16_t*>(&b);
+      v -= __half2float(b);
+    }
+  }
+  return make_uint4(h[0] | (h[1] << 16), h[2], 0u, 0u);
+}
+
+// delta = rowsum(dO * O), LPR lanes per row (as many as the row has 16-byte chunks, so that every lane
+// of the warp loads), each lane keeping the loads of kDeltaRows rows in flight.  When `zero` is given, the
+// warp also clears zero_vec_per_row float4 per row of it -- the fused backward's f32 dQ accumulator, by
+// the pass that already streams O and dO -- and with `aux_lse` it writes the folded operands of its rows.
+// Bound by memory.  64 heads x 8192 rows, D = 64 (285 MB): 96 us with a warp per row, three quarters of
+// its lanes idle, and the folded operands in a pass of their own; 49 us (5.9 TB/s) like this.  32 heads x
+// 4096 rows, D = 128 (134 MB): 27 -> 20 us.
 constexpr int kDeltaRows = 4;
 
-template <bool BF16>
+struct FoldOut {
+  const float* lse;
+  uint4* aux_lse;    // null: nothing to fold
+  uint4* aux_delta;
+  float mask_value;
+};
+
+template <int LPR, bool BF16>
 __global__ void __launch_bounds__(256) delta_kernel(const uint4* __restrict__ o, const uint4* __restrict__ d_out,
                                                     float* __restrict__ delta, long long rows, int chunks_per_row,
-                                                    float4* __restrict__ zero, int zero_vec_per_row) {
-  const long long row0 = (static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * kDeltaRows;
-  const int lane = threadIdx.x & 31;
-  if (row0 >= rows) return;
+                                                    float4* __restrict__ zero, int zero_vec_per_row, const FoldOut fold) {
+  constexpr int kRowsAtOnce = 32 / LPR;
+  constexpr int kWarpRows = kRowsAtOnce * kDeltaRows;
+  const int lane = threadIdx.x & 31, sub = lane % LPR, which = lane / LPR;
+  const long long warp_row0 = (static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * kWarpRows;
+  if (warp_row0 >= rows) return;
+  const long long row0 = warp_row0 + which;  // this lane's rows: row0 + r * kRowsAtOnce
   float acc[kDeltaRows];
 #pragma unroll
   for (int r = 0; r < kDeltaRows; ++r) acc[r] = 0.f;
-  for (int c = lane; c < chunks_per_row; c += 32) {
+  for (int c = sub; c < chunks_per_row; c += LPR) {
     uint4 a[kDeltaRows], b[kDeltaRows];
 #pragma unroll
     for (int r = 0; r < kDeltaRows; ++r) {
-      const bool live = row0 + r < rows;
-      a[r] = live ? o[(row0 + r) * chunks_per_row + c] : make_uint4(0, 0, 0, 0);
-      b[r] = live ? d_out[(row0 + r) * chunks_per_row + c] : make_uint4(0, 0, 0, 0);
+      const long long row = row0 + r * kRowsAtOnce;
+      const bool live = row < rows;
+      a[r] = live ? o[row * chunks_per_row + c] : make_uint4(0, 0, 0, 0);
+      b[r] = live ? d_out[row * chunks_per_row + c] : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int r = 0; r < kDeltaRows; ++r) {
@@ -60,33 +97,49 @@ __global__ void __launch_bounds__(256) delta_kernel(const uint4* __restrict__ o,
   }
   if (zero) {
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int r = 0; r < kDeltaRows; ++r)
-      if (row0 + r < rows)
-        for (int c = lane; c < zero_vec_per_row; c += 32) zero[(row0 + r) * zero_vec_per_row + c] = z;
+    const long long left = rows - warp_row0;
+    const int vecs = static_cast<int>(left < kWarpRows ? left : kWarpRows) * zero_vec_per_row;
+    float4* dst = zero + warp_row0 * zero_vec_per_row;
+    for (int c = lane; c < vecs; c += 32) dst[c] = z;
   }
 #pragma unroll
   for (int r = 0; r < kDeltaRows; ++r) {
     float v = acc[r];
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-    if (lane == 0 && row0 + r < rows) delta[row0 + r] = v;
+    for (int s = LPR / 2; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
+    const long long row = row0 + r * kRowsAtOnce;
+    if (row < rows) {
+      if (sub == 0) {
+        delta[row] = v;
+        if (fold.aux_lse) fold.aux_delta[row] = split3_neg<BF16>(v, false);
+      } else if (sub == 1 && fold.aux_lse) {
+        const float l = fold.lse[row];
+        fold.aux_lse[row] = split3_neg<BF16>(l, l == fold.mask_value);
+      }
+    }
   }
 }
 
+template <int LPR>
+static void run_delta(const void* o, const void* d_out, float* delta, long long rows, int chunks, int dtype,
+                      cudaStream_t stream, float* zero, int zero_floats_per_row, const FoldOut& fold) {
+  constexpr int kBlockRows = 8 * (32 / LPR) * kDeltaRows;
+  const unsigned grid = static_cast<unsigned>((rows + kBlockRows - 1) / kBlockRows);
+  auto kernel = dtype == SPLASH_DTYPE_BF16 ? delta_kernel<LPR, true> : delta_kernel<LPR, false>;
+  kernel<<<grid, 256, 0, stream>>>(static_cast<const uint4*>(o), static_cast<const uint4*>(d_out), delta, rows, chunks,
+                                   reinterpret_cast<float4*>(zero), zero_floats_per_row / 4, fold);
+}
+
 int launch_delta(const void* o, const void* d_out, float* delta, long long rows, int head_dim_v, int dtype,
-                 cudaStream_t stream, float* zero, int zero_floats_per_row) {
+                 cudaStream_t stream, float* zero, int zero_floats_per_row, const float* lse, void* aux_lse,
+                 void* aux_delta, float mask_value) {
   if (!o || !d_out || !delta || rows <= 0 || head_dim_v % 8) return fail(SPLASH_INVALID_ARGUMENT, "bad delta arguments");
   if (zero && zero_floats_per_row % 4) return fail(SPLASH_INVALID_ARGUMENT, "bad delta arguments");
-  const unsigned grid = static_cast<unsigned>((rows + 8 * kDeltaRows - 1) / (8 * kDeltaRows));
-  if (dtype == SPLASH_DTYPE_BF16)
-    delta_kernel<true><<<grid, 256, 0, stream>>>(static_cast<const uint4*>(o), static_cast<const uint4*>(d_out), delta,
-                                                  rows, head_dim_v / 8, reinterpret_cast<float4*>(zero),
-                                                  zero_floats_per_row / 4);
-  else
-    delta_kernel<false><<<grid, 256, 0, stream>>>(static_cast<const uint4*>(o), static_cast<const uint4*>(d_out), delta,
-                                                   rows, head_dim_v / 8, reinterpret_cast<float4*>(zero),
-                                                   zero_floats_per_row / 4);
+  const int chunks = head_dim_v / 8;
+  const FoldOut fold{lse, static_cast<uint4*>(aux_lse), static_cast<uint4*>(aux_delta), mask_value};
+  if (chunks == 8) run_delta<8>(o, d_out, delta, rows, chunks, dtype, stream, zero, zero_floats_per_row, fold);
+  else if (chunks == 16) run_delta<16>(o, d_out, delta, rows, chunks, dtype, stream, zero, zero_floats_per_row, fold);
+  else run_delta<32>(o, d_out, delta, rows, chunks, dtype, stream, zero, zero_floats_per_row, fold);
   SPLASH_CUDA_CHECK(cudaGetLastError());
   return SPLASH_OK;
 }
@@ -126,29 +179,6 @@ __global__ void __launch_bounds__(256) dq_transpose_cast_kernel(const float* __r
     }
     *reinterpret_cast<uint32_t*>(dst + static_cast<long long>(q) * head_dim + 2 * lane) = w;
   }
-}
-
-// Splits -x into three 16-bit floats whose sum is -x to f32 precision, as the eight 16-bit
-// values {hi, mid, lo, 0, 0, 0, 0, 0} per row that the 128-row fused backward (head_dim 64)
-// multiplies by {1, 1, 1, 0, ...} in one extra K = 16 slice of its score products.  Rows whose
-// lse is mask_value (they saw no key) get a large negative value instead, which makes their P zero.
-template <bool BF16>
-__device__ __forceinline__ uint4 split3_neg(float x, bool sentinel) {
-  float v = sentinel ? (BF16 ? -1.0e30f : -60000.f) : -x;
-  uint32_t h[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    if constexpr (BF16) {
-      const __nv_bfloat16 b = __float2bfloat16_rn(v);
-      h[i] = *reinterpret_cast<const uint16_t*>(&b);
-      v -= __bfloat162float(b);
-    } else {
-      const __half b = __float2half_rn(v);
-      h[i] = *reinterpret_cast<const uint16_t*>(&b);
-      v -= __half2float(b);
-    }
-  }
-  return make_uint4(h[0] | (h[1] << 16), h[2], 0u, 0u);
 }
 
 template <bool BF16>

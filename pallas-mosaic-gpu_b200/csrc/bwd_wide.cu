@@ -31,14 +31,8 @@ static int launch_bwd_wide_typed(const SplashParams& p, cudaStream_t stream) {
   BwdArgs a;
   fill_bwd_args(a, p, p.partial_blocks != nullptr, seg);
   a.stages = L::kSlots;
-  if (L::kFold) {
-    // The scratch holds the f32 dQ accumulator, then the folded -lse and -delta operands.
-    const long long rows = static_cast<long long>(p.batch) * p.heads * p.q_len;
-    uint8_t* aux = reinterpret_cast<uint8_t*>(p.dq_acc) + rows * D * 4;
-    a.aux_lse = aux;
-    a.aux_delta = aux + rows * 16;
-    if ((rc = launch_fold_operands(p.lse, p.delta, aux, aux + rows * 16, rows, p.mask_value, p.dtype, stream))) return rc;
-  }
+  a.aux_lse = fold_operand_lse(p);  // filled by the caller
+  a.aux_delta = fold_operand_delta(p);
   // Segment skipping when the CTA's list of block steps fits the room set aside for it.
   const bool skipping = seg && p.seg_ranges != nullptr && (p.heads / p.kv_heads) * p.max_steps <= L::kListSteps;
   a.seg_q_ranges = skipping ? seg_q_ranges(p) : nullptr;

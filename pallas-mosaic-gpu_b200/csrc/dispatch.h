@@ -28,9 +28,11 @@ size_t bwd_row_smem(const SplashParams& p);
 int launch_bwd_wide(const SplashParams& p, cudaStream_t stream);
 
 // delta = rowsum(dO * O); dq = cast(dq_acc), transposed where the accumulator is.
-// When `zero` is non-null the same pass also clears zero_floats_per_row floats per row of it.
+// When `zero` is non-null the same pass also clears zero_floats_per_row floats per row of it, and when
+// `aux_lse` is, it does what launch_fold_operands does.
 int launch_delta(const void* o, const void* d_out, float* delta, long long rows, int head_dim_v, int dtype,
-                 cudaStream_t stream, float* zero = nullptr, int zero_floats_per_row = 0);
+                 cudaStream_t stream, float* zero = nullptr, int zero_floats_per_row = 0, const float* lse = nullptr,
+                 void* aux_lse = nullptr, void* aux_delta = nullptr, float mask_value = 0.f);
 int launch_dq_cast(const float* acc, void* dq, long long batch_heads, int head_dim, int q_len, int dtype,
                    cudaStream_t stream);
 // -lse and -delta of every q row as three 16-bit parts each (16 bytes per row and array): the
@@ -38,8 +40,17 @@ int launch_dq_cast(const float* acc, void* dq, long long batch_heads, int head_d
 int launch_fold_operands(const float* lse, const float* delta, void* aux_lse, void* aux_delta, long long rows,
                          float mask_value, int dtype, cudaStream_t stream);
 // Bytes of those two arrays together (they follow the f32 dQ accumulator in the fused backward's scratch).
+inline long long q_row_count(const SplashParams& p) { return static_cast<long long>(p.batch) * p.heads * p.q_len; }
 inline long long fold_operand_bytes(const SplashParams& p) {
   return p.head_dim == 64 ? 2ll * 16 * p.batch * p.heads * p.q_len : 0;
+}
+
+// ... and where they lie: -lse first, -delta behind it (null at head_dim 128, which folds nothing).
+inline uint8_t* fold_operand_lse(const SplashParams& p) {
+  return p.head_dim == 64 ? reinterpret_cast<uint8_t*>(p.dq_acc) + q_row_count(p) * p.head_dim * 4 : nullptr;
+}
+inline uint8_t* fold_operand_delta(const SplashParams& p) {
+  return p.head_dim == 64 ? fold_operand_lse(p) + q_row_count(p) * 16 : nullptr;
 }
 
 // Fills p.seg_ranges (when given, with segment ids) with the (min, max) id of every 64 positions.
