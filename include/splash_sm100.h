@@ -181,6 +181,12 @@ int splash_bwd_fused_static(const SplashParams* p, void* stream);
  * SPLASH_OK, SPLASH_DEVICE_TIMEOUT or SPLASH_CUDA_ERROR. `host_out` may be NULL. */
 int splash_read_status(const int32_t* status, int32_t* host_out, void* stream);
 
+/* Queues a copy of the status word to pinned host memory behind what `stream` holds, without waiting:
+ * records `launched` on `stream`, makes `side_stream` wait for it, copies there and records `copied`
+ * (two cudaEvent_t of the caller).  Not during stream capture. */
+int splash_status_copy(const int32_t* status, int32_t* host, void* stream, void* side_stream, void* launched,
+                       void* copied);
+
 /* Human-readable text for a SplashStatus value (static storage). */
 const char* splash_status_string(int status);
 

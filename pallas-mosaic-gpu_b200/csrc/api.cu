@@ -229,6 +229,18 @@ extern "C" int splash_read_status(const int32_t* status, int32_t* host_out, void
   return SPLASH_OK;
 }
 
+extern "C" int splash_status_copy(const int32_t* status, int32_t* host, void* stream, void* side_stream, void* launched,
+                                  void* copied) {
+  if (!status || !host || !side_stream || !launched || !copied)
+    return fail(SPLASH_INVALID_ARGUMENT, "splash_status_copy needs the word, its host copy, a side stream and two events");
+  cudaStream_t side = static_cast<cudaStream_t>(side_stream);
+  SPLASH_CUDA_CHECK(cudaEventRecord(static_cast<cudaEvent_t>(launched), static_cast<cudaStream_t>(stream)));
+  SPLASH_CUDA_CHECK(cudaStreamWaitEvent(side, static_cast<cudaEvent_t>(launched), 0));
+  SPLASH_CUDA_CHECK(cudaMemcpyAsync(host, status, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, side));
+  SPLASH_CUDA_CHECK(cudaEventRecord(static_cast<cudaEvent_t>(copied), side));
+  return SPLASH_OK;
+}
+
 extern "C" const char* splash_status_string(int status) {
   switch (status) {
     case SPLASH_OK: return "ok";

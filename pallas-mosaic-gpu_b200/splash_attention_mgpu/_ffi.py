@@ -39,6 +39,7 @@ EXPORTED_SYMBOLS = (
     "splash_bwd_fused_static",
     "splash_seg_ranges_bytes",
     "splash_read_status",
+    "splash_status_copy",
     "splash_status_string",
     "splash_last_error",
     "splash_selftest_umma",
@@ -106,6 +107,8 @@ def load():
     lib.splash_bwd_fused_workspace_bytes.restype = c_int64
   lib.splash_read_status.argtypes = [c_void_p, POINTER(c_int32 * 4), c_void_p]
   lib.splash_read_status.restype = c_int
+  lib.splash_status_copy.argtypes = [c_void_p] * 6
+  lib.splash_status_copy.restype = c_int
   lib.splash_status_string.argtypes = [c_int]
   lib.splash_status_string.restype = c_char_p
   lib.splash_last_error.argtypes = []

@@ -21,6 +21,7 @@ without a CUDA device a call raises.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import dataclasses
 import functools
@@ -45,9 +46,28 @@ _TORCH_DTYPES = {torch.bfloat16: _ffi.DTYPE_BF16, torch.float16: _ffi.DTYPE_F16}
 # ---------------------------------------------------------------------------
 
 _status_words: dict = {}
-# device key -> (pinned host copy of the word, event recorded after the copy, side stream that carries
-# the copy, event that marks the kernels the copy has to follow)
-_status_mirrors: dict = {}
+_status_mirrors: dict = {}  # device key -> _StatusMirror
+
+
+class _StatusMirror:
+  """Pinned host copy of a device's status word and what carries the copy: a side stream, the event that
+  marks the kernels the copy follows, and the event recorded behind it."""
+
+  def __init__(self, device):
+    self.host = torch.zeros(4, dtype=torch.int32).pin_memory()
+    self.code = ctypes.c_int32.from_address(self.host.data_ptr())
+    self.side, self.launched, self.copied = torch.cuda.Stream(device), torch.cuda.Event(), torch.cuda.Event()
+    with torch.cuda.device(device):
+      for event in (self.launched, self.copied):  # an event gets its handle when it is first recorded
+        event.record(self.side)
+    # Raw handles: the copy is queued by one call into the library.
+    self.handles = (self.side.cuda_stream, self.launched.cuda_event, self.copied.cuda_event)
+
+  def reset(self):
+    """Forgets what was copied, once no copy is on its way any more.  (The object stays: a copy queued by
+    the library is unknown to the allocator of pinned memory, which must not hand the buffer on under it.)"""
+    self.copied.synchronize()
+    self.host.zero_()
 
 
 def _status_word(device: torch.device) -> torch.Tensor:
@@ -56,6 +76,15 @@ def _status_word(device: torch.device) -> torch.Tensor:
   if key not in _status_words:
     _status_words[key] = torch.zeros(4, dtype=torch.int32, device=device)
   return _status_words[key]
+
+
+def _on_device(device: torch.device):
+  """Makes `device` the current one for a block; costs next to nothing where it is already."""
+  return contextlib.nullcontext() if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
+def _raw_stream(device: torch.device) -> int:
+  return torch._C._cuda_getCurrentRawStream(device.index)  # what current_stream(device).cuda_stream wraps
 
 
 def _raise_device_status(word: torch.Tensor, host) -> None:
@@ -78,7 +107,8 @@ def check_device_status(device=None) -> None:
     with torch.cuda.device(word.device):
       stream = torch.cuda.current_stream(word.device).cuda_stream
       rc = lib.splash_read_status(word.data_ptr(), ctypes.byref(host), stream)
-    _status_mirrors.pop(key, None)
+    if key in _status_mirrors:
+      _status_mirrors[key].reset()
     if rc == _ffi.SPLASH_DEVICE_TIMEOUT:
       _raise_device_status(word, host)
     _ffi.check(rc, "splash attention kernel")
@@ -88,12 +118,12 @@ def _poll_status(device) -> None:
   """Start of a call: raises if the copy queued by an earlier call has landed and shows a failure.
   Never waits for the device."""
   mirror = _status_mirrors.get((device.type, device.index))
-  if mirror is None or torch.cuda.is_current_stream_capturing():
+  if mirror is None or mirror.code.value == 0 or torch.cuda.is_current_stream_capturing():
     return
-  host, event = mirror[:2]
-  if event.query() and int(host[0]) != 0:
-    _status_mirrors.pop((device.type, device.index), None)
-    _raise_device_status(_status_word(device), host.tolist())
+  if mirror.copied.query():
+    record = mirror.host.tolist()
+    mirror.reset()
+    _raise_device_status(_status_word(device), record)
 
 
 def _maybe_check(device) -> None:
@@ -112,15 +142,11 @@ def _maybe_check(device) -> None:
   key = (device.type, device.index)
   mirror = _status_mirrors.get(key)
   if mirror is None:
-    mirror = (torch.zeros(4, dtype=torch.int32).pin_memory(), torch.cuda.Event(), torch.cuda.Stream(device),
-              torch.cuda.Event())
-    _status_mirrors[key] = mirror
-  host, event, side, launched = mirror
-  launched.record(torch.cuda.current_stream(device))
-  side.wait_event(launched)
-  with torch.cuda.stream(side):
-    host.copy_(_status_word(device), non_blocking=True)
-    event.record(side)
+    mirror = _status_mirrors[key] = _StatusMirror(device)
+  with _on_device(device):
+    rc = _ffi.load().splash_status_copy(_status_word(device).data_ptr(), mirror.host.data_ptr(), _raw_stream(device),
+                                        *mirror.handles)
+  _ffi.check(rc, "splash attention status copy")
 
 
 class _DeviceSchedule(NamedTuple):
@@ -224,6 +250,7 @@ class SplashAttentionKernel:
     self.interpret = interpret
     self._infos: dict = {}
     self._device_schedules: dict = {}
+    self._resolved: dict = {}
 
   @property
   def info(self) -> mask_info_lib.GpuMaskInfo:
@@ -289,6 +316,15 @@ class SplashAttentionKernel:
       return bs.block_q
     return self._auto_forward_tiling(head_dim, head_dim_v, **kw)[0]
 
+  def _call_block_sizes(self, head_dim: int, head_dim_v: int, itemsize: int, has_segments: bool) -> BlockSizes:
+    """`resolved_block_sizes` of a call, worked out once per class of calls."""
+    key = (self.requested_block_sizes, head_dim, head_dim_v, itemsize, has_segments)
+    bs = self._resolved.get(key)
+    if bs is None:
+      bs = self._resolved[key] = self.resolved_block_sizes(head_dim, head_dim_v, itemsize=itemsize,
+                                                           has_segments=has_segments)
+    return bs
+
   def resolved_block_sizes(self, head_dim: int, head_dim_v: int, **kw) -> BlockSizes:
     bs = self.requested_block_sizes
     if bs.block_q is None:
@@ -327,9 +363,8 @@ class SplashAttentionKernel:
       raise NotImplementedError(
           "interpret= selects the reference's CPU interpreter; this library"
           " only runs on an sm_100a GPU.")
-    bs = self.resolved_block_sizes(
-        q.shape[-1], v.shape[-1], itemsize=q.element_size(),
-        has_segments=segment_ids is not None)
+    bs = self._call_block_sizes(
+        q.shape[-1], v.shape[-1], q.element_size(), segment_ids is not None)
     return _splash_attention(self, bs, q, k, v, segment_ids,
                              save_residuals=save_residuals)
 
@@ -501,8 +536,8 @@ def _forward(kernel: SplashAttentionKernel, bs: BlockSizes, q, k, v,
   p = _base_params(kernel, q, k, v, segment_ids, sched)
   p.out, p.lse_out = out.data_ptr(), _ptr(lse)
   p.block_q, p.block_kv, p.num_stages = bs.block_q, bs.block_kv, bs.num_stages
-  with torch.cuda.device(q.device):
-    stream = torch.cuda.current_stream(q.device).cuda_stream
+  with _on_device(q.device):
+    stream = _raw_stream(q.device)
     entry = lib.splash_fwd256 if bs.block_q == cfg.PINGPONG_ROWS else lib.splash_fwd128
     _ffi.check(entry(ctypes.byref(p), stream), "splash attention forward")
   _maybe_check(q.device)
@@ -554,8 +589,8 @@ def _backward(kernel: SplashAttentionKernel, bs: BlockSizes, q, k, v,
   dk = torch.empty_like(k)
   dv = torch.empty_like(v)
   fused = _use_fused_backward(q, v, bs, has_dense, has_segments)
-  with torch.cuda.device(q.device):
-    stream = torch.cuda.current_stream(q.device).cuda_stream
+  with _on_device(q.device):
+    stream = _raw_stream(q.device)
     if not fused:
       _ffi.check(lib.splash_bwd_delta(out.data_ptr(), d_out.data_ptr(),
                                       delta.data_ptr(), batch * heads * q_len,
