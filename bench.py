@@ -661,8 +661,8 @@ def run_ours(args):
           continue
         uq, uk, uv, _ = (x.to(dev) for x in part.host_inputs(pin=False, span=(lo, lo + 1)))
         useg = part.segment_ids(sa, dev, span=(lo, lo + 1))
-        with torch.no_grad():
-          mine = kernel(uq, uk, uv, useg)
+        # As in the step: calls that gradients follow do not tile by how much is in the call.
+        mine = kernel(uq.requires_grad_(True), uk, uv, useg).detach()
         same = same and bool(torch.equal(mine[0], units[lo]))
         n_checked += 1
       check = dict(gathered_units=int(units.shape[0]), recomputed_on_rank0=n_checked, bit_identical=same,

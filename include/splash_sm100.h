@@ -117,6 +117,13 @@ int splash_fwd128(const SplashParams* p, void* stream);
  * (reference splash_attention_mgpu/forward_pingpong.py:667-681). */
 int splash_fwd256(const SplashParams* p, void* stream);
 
+/* Forward with several CTAs per q tile where one per tile would leave SMs idle (few tiles, long
+ * rows); block_q selects the kernel (128 or 256).  splash_fwd_split_bytes() says how many bytes of
+ * `workspace` (16-byte aligned) the shares of these shapes need on the current device; 0: the call
+ * does what splash_fwd128 / splash_fwd256 does and needs none.  No counterpart in the reference. */
+int64_t splash_fwd_split_bytes(const SplashParams* p);
+int splash_fwd_split(const SplashParams* p, void* workspace, int64_t bytes, void* stream);
+
 /* delta = rowsum(dO * O) in f32, the reduction the reference leaves to XLA
  * (reference splash_attention_mgpu/splash_attention.py:289-290).
  * `o` and `d_out` are [rows, head_dim_v] of `dtype`; `delta` is [rows] f32. */

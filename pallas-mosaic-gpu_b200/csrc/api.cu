@@ -45,7 +45,8 @@ static int check_fwd(const SplashParams* p, int tiles) {
 
 #define SPLASH_FWD_CASE(D_, DV_, NT_)                                                               \
   if (p->head_dim == D_ && p->head_dim_v == DV_) {                                                  \
-    return p->block_kv == 64 ? launch_fwd<D_, DV_, 64, NT_>(*p, st) : launch_fwd<D_, DV_, 128, NT_>(*p, st); \
+    return p->block_kv == 64 ? launch_fwd<D_, DV_, 64, NT_>(*p, splits, ws, st)                      \
+                             : launch_fwd<D_, DV_, 128, NT_>(*p, splits, ws, st);                    \
   }
 
 }  // namespace splash
@@ -57,9 +58,8 @@ extern "C" int64_t splash_seg_ranges_bytes(const SplashParams* p) {
   return static_cast<int64_t>(p->batch) * (p->q_len / 64 + p->kv_len / 64) * 8;
 }
 
-extern "C" int splash_fwd128(const SplashParams* p, void* stream) {
+static int fwd128(const SplashParams* p, int splits, void* ws, cudaStream_t st) {
   if (int rc = check_fwd(p, 1)) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (int rc = launch_seg_ranges(*p, st)) return rc;
   SPLASH_FWD_CASE(64, 64, 1)
   SPLASH_FWD_CASE(64, 128, 1)
@@ -70,14 +70,56 @@ extern "C" int splash_fwd128(const SplashParams* p, void* stream) {
   return fail(SPLASH_UNSUPPORTED, "this (head_dim, head_dim_v) pair is not compiled for the 128-row forward");
 }
 
-extern "C" int splash_fwd256(const SplashParams* p, void* stream) {
+static int fwd256(const SplashParams* p, int splits, void* ws, cudaStream_t st) {
   if (int rc = check_fwd(p, 2)) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (int rc = launch_seg_ranges(*p, st)) return rc;
   if (p->head_dim != p->head_dim_v) return fail(SPLASH_UNSUPPORTED, "ping-pong kernel needs head_dim == head_dim_v");
   SPLASH_FWD_CASE(64, 64, 2)
   SPLASH_FWD_CASE(128, 128, 2)
   return fail(SPLASH_UNSUPPORTED, "ping-pong kernel supports head_dim 64/128");
+}
+
+extern "C" int splash_fwd128(const SplashParams* p, void* stream) {
+  return fwd128(p, 1, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int splash_fwd256(const SplashParams* p, void* stream) {
+  return fwd256(p, 1, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+// CTAs per q tile that fill the GPU once.  A grid of one CTA per tile leaves SMs idle when tiles are few
+// (a chunk of queries against a long cache, small batches), and the heaviest tile then sets the time.
+// Shares of fewer than 512 keys are not made, and at least 2048 keys have to come off the longest tile:
+// the combining pass and its launch cost what about that many do.
+static int fwd_splits(const SplashParams* p) {
+  if (!p || p->block_q <= 0 || p->q_len <= 0 || p->batch <= 0 || p->heads <= 0) return 1;
+  const bool two_per_sm = p->block_q == 128 && p->block_kv == 64 && p->head_dim <= 128 && p->head_dim_v <= 128;
+  const int64_t slots = static_cast<int64_t>(sm_count()) * (two_per_sm ? 2 : 1);
+  const int64_t tiles = static_cast<int64_t>(p->q_len / p->block_q) * p->heads * p->batch;
+  if (tiles <= 0) return 1;
+  const int64_t keys = static_cast<int64_t>(p->max_steps) * p->block_kv;
+  int64_t splits = slots / tiles;
+  if (splits > keys / 512) splits = keys / 512;
+  if (splits > 32) splits = 32;
+  if (splits < 2 || keys - keys / splits < 2048) return 1;
+  return static_cast<int>(splits);
+}
+
+extern "C" int64_t splash_fwd_split_bytes(const SplashParams* p) {
+  const int splits = fwd_splits(p);
+  if (splits < 2) return 0;
+  return splits * q_row_count(*p) * (static_cast<int64_t>(p->head_dim_v) * 4 + 8);
+}
+
+extern "C" int splash_fwd_split(const SplashParams* p, void* workspace, int64_t bytes, void* stream) {
+  const int splits = fwd_splits(p);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool two_tiles = p && p->block_q == 256;
+  if (splits < 2) return two_tiles ? fwd256(p, 1, nullptr, st) : fwd128(p, 1, nullptr, st);
+  if (!workspace || bytes < splash_fwd_split_bytes(p) || (reinterpret_cast<uintptr_t>(workspace) & 15))
+    return fail(SPLASH_INVALID_ARGUMENT, "the workspace of a split forward is null, too small or not 16-byte aligned");
+  if (int rc = two_tiles ? fwd256(p, splits, workspace, st) : fwd128(p, splits, workspace, st)) return rc;
+  return launch_fwd_combine(*p, splits, workspace, st);
 }
 
 static int check_bwd(const SplashParams* p) {

@@ -8,8 +8,9 @@
 
 namespace splash {
 
+// `splits` CTAs per q tile; above 1 they leave their parts in `workspace` (see launch_fwd_combine).
 template <int D, int DV, int BKV, int NT>
-int launch_fwd(const SplashParams& p, cudaStream_t stream);
+int launch_fwd(const SplashParams& p, int splits, void* workspace, cudaStream_t stream);
 
 }  // namespace splash
 
@@ -23,6 +24,9 @@ int launch_bwd_row(const SplashParams& p, cudaStream_t stream);
 
 template <int D, int DV, int BC>
 size_t bwd_row_smem(const SplashParams& p);
+
+// Puts the parts of a split forward together: out and, when asked for, lse.
+int launch_fwd_combine(const SplashParams& p, int splits, const void* workspace, cudaStream_t stream);
 
 // Fused backward, 128 q rows per step (head_dim == head_dim_v, 64 or 128).
 int launch_bwd_wide(const SplashParams& p, cudaStream_t stream);

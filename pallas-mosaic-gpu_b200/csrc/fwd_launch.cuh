@@ -9,8 +9,8 @@
 
 namespace splash {
 
-template <int D, int DV, int BKV, int NT, int AW, bool PLAIN, bool BF16>
-int launch_fwd_plain(const SplashParams& p, cudaStream_t stream) {
+template <int D, int DV, int BKV, int NT, int AW, bool PLAIN, bool SPLIT, bool BF16>
+int launch_fwd_plain(const SplashParams& p, int splits, void* workspace, cudaStream_t stream) {
   using L = FwdLayout<D, DV, BKV, NT, AW>;
   const bool dense = p.partial_blocks != nullptr;
   const bool seg = p.seg_q != nullptr;
@@ -68,10 +68,13 @@ int launch_fwd_plain(const SplashParams& p, cudaStream_t stream) {
   a.head_group = 8;
   a.mask_value = p.mask_value;
   a.soft_cap = p.soft_cap;
+  a.splits = splits;
+  a.part_o = static_cast<float*>(workspace);
+  a.part_ml = splits > 1 ? reinterpret_cast<float2*>(a.part_o + static_cast<size_t>(splits) * q_rows * DV) : nullptr;
 
-  auto kernel = splash_fwd_kernel<D, DV, BKV, NT, AW, PLAIN, BF16>;
+  auto kernel = splash_fwd_kernel<D, DV, BKV, NT, AW, PLAIN, SPLIT, BF16>;
   if ((rc = opt_in_smem(kernel, smem))) return rc;
-  const unsigned grid = static_cast<unsigned>(a.q_blocks) * p.heads * p.batch;
+  const unsigned grid = static_cast<unsigned>(a.q_blocks) * p.heads * p.batch * splits;
   kernel<<<grid, L::kThreads, smem, stream>>>(tm_q, tm_k, tm_v, tm_o, a);
   SPLASH_CUDA_CHECK(cudaGetLastError());
   return SPLASH_OK;
@@ -79,10 +82,13 @@ int launch_fwd_plain(const SplashParams& p, cudaStream_t stream) {
 
 // The kernel without its soft-cap, segment and streamed-mask code when the call uses none.
 template <int D, int DV, int BKV, int NT, int AW, bool BF16>
-int launch_fwd_typed(const SplashParams& p, cudaStream_t stream) {
+int launch_fwd_typed(const SplashParams& p, int splits, void* workspace, cudaStream_t stream) {
   const bool plain = p.soft_cap == 0.f && p.seg_q == nullptr && p.partial_blocks == nullptr;
-  if (plain) return launch_fwd_plain<D, DV, BKV, NT, AW, true, BF16>(p, stream);
-  return launch_fwd_plain<D, DV, BKV, NT, AW, false, BF16>(p, stream);
+  if (splits > 1)
+    return plain ? launch_fwd_plain<D, DV, BKV, NT, AW, true, true, BF16>(p, splits, workspace, stream)
+                 : launch_fwd_plain<D, DV, BKV, NT, AW, false, true, BF16>(p, splits, workspace, stream);
+  return plain ? launch_fwd_plain<D, DV, BKV, NT, AW, true, false, BF16>(p, splits, workspace, stream)
+               : launch_fwd_plain<D, DV, BKV, NT, AW, false, false, BF16>(p, splits, workspace, stream);
 }
 
 // Softmax warpgroups per q tile of the one-tile kernel.  Two that alternate over the KV steps where
@@ -100,11 +106,11 @@ constexpr int fwd_softmax_groups() {
 }
 
 template <int D, int DV, int BKV, int NT>
-int launch_fwd(const SplashParams& p, cudaStream_t stream) {
+int launch_fwd(const SplashParams& p, int splits, void* workspace, cudaStream_t stream) {
   const bool bf16 = p.dtype == SPLASH_DTYPE_BF16;
   constexpr int AW = fwd_softmax_groups<DV, BKV, NT>();
-  if (bf16) return launch_fwd_typed<D, DV, BKV, NT, AW, true>(p, stream);
-  return launch_fwd_typed<D, DV, BKV, NT, AW, false>(p, stream);
+  if (bf16) return launch_fwd_typed<D, DV, BKV, NT, AW, true>(p, splits, workspace, stream);
+  return launch_fwd_typed<D, DV, BKV, NT, AW, false>(p, splits, workspace, stream);
 }
 
 }  // namespace splash

@@ -95,6 +95,16 @@ inline int opt_in_smem(Kernel kernel, size_t bytes) {
   return opt_in_smem_impl(reinterpret_cast<const void*>(kernel), bytes);
 }
 
+// SMs of the current device (the library is built for one GPU model: asked once).
+inline int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    return v;
+  }();
+  return n;
+}
+
 constexpr size_t kMaxDynamicSmem = 227 * 1024;
 
 }  // namespace splash

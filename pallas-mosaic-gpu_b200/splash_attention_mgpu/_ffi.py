@@ -31,6 +31,8 @@ DTYPE_F16 = 1
 EXPORTED_SYMBOLS = (
     "splash_fwd128",
     "splash_fwd256",
+    "splash_fwd_split",
+    "splash_fwd_split_bytes",
     "splash_bwd_delta",
     "splash_bwd_dq",
     "splash_bwd_dkv",
@@ -99,6 +101,10 @@ def load():
     lib.splash_bwd_delta.argtypes = [c_void_p, c_void_p, c_void_p, c_int64,
                                      c_int32, c_int32, c_void_p]
     lib.splash_bwd_delta.restype = c_int
+  lib.splash_fwd_split.argtypes = [POINTER(SplashParams), c_void_p, c_int64, c_void_p]
+  lib.splash_fwd_split.restype = c_int
+  lib.splash_fwd_split_bytes.argtypes = [POINTER(SplashParams)]
+  lib.splash_fwd_split_bytes.restype = c_int64
   if hasattr(lib, "splash_seg_ranges_bytes"):
     lib.splash_seg_ranges_bytes.argtypes = [POINTER(SplashParams)]
     lib.splash_seg_ranges_bytes.restype = c_int64

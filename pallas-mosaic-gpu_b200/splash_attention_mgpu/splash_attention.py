@@ -25,6 +25,7 @@ import contextlib
 import ctypes
 import dataclasses
 import functools
+import math
 import os
 from typing import Any, NamedTuple
 
@@ -273,7 +274,8 @@ class SplashAttentionKernel:
 
   def _auto_forward_tiling(self, head_dim: int, head_dim_v: int, *,
                            itemsize: int = 2, has_segments: bool = False,
-                           save_residuals: bool = True) -> tuple[int, int, int]:
+                           save_residuals: bool = True,
+                           tiles: int | None = None) -> tuple[int, int, int]:
     """(block_q, block_kv, num_stages) when the caller left block_q open.
 
     At head_dim 128 the one-tile kernel serves every mask measured on B200 at
@@ -283,7 +285,24 @@ class SplashAttentionKernel:
     softmax warpgroups alternating over the KV steps for long rows.  The
     two-tile kernel (block_q=256) runs when asked for, and at head_dim 64 on masks
     whose 256-row schedule costs nothing extra.
+
+    `tiles` is the call's number of 128-row q tiles over batch and heads.  Up to one per SM the second
+    CTA that 64-wide blocks leave room for has no tile, and 128-wide blocks with their two softmax
+    warpgroups are faster at any row length (causal, D = 128: 8 heads, seq 1024 21.3 -> 18.4 us, 4 heads,
+    seq 4096 53 -> 38 us; D = 64: 2 heads, seq 4096 49 -> 37 us).  Up to one and three quarters per SM that
+    still holds where the rows differ in length as under a causal mask, for the two CTAs that share an SM
+    then hold up its longest row (192 tiles, seq 2048: 36.9 -> 28.7 us; 256 tiles, seq 4096: 59 -> 44 us; at
+    288 tiles 41.0 against 41.8), but not where they are alike (local, 192 tiles: 23.5 against 26.6 us).
     """
+    if (tiles is not None and head_dim == head_dim_v and head_dim in (64, 128)
+        and tiles <= cfg.FEW_TILES[1]):
+      info = self.fwd_info(128, 128)
+      few = dict(head_dim=head_dim, head_dim_v=head_dim_v, block_kv=128, num_stages=2, itemsize=itemsize,
+                 has_dense_mask=info.partial_mask_blocks is not None,
+                 has_segments=has_segments, save_residuals=save_residuals)
+      uneven = float(info.num_steps.mean()) <= 0.6 * float(info.num_steps.max())
+      if (tiles <= cfg.FEW_TILES[0] or uneven) and cfg.fwd128_smem_bytes(**few) <= cfg.SMEM_BYTES:
+        return 128, 128, 2
     if head_dim == head_dim_v == 64:
       # Measured at seq 8192 (tuning.py): 64-wide KV blocks with a two-stage ring (two CTAs per SM)
       # lead on causal-like masks; the two-tile kernel leads where its 256-row schedule visits no
@@ -316,17 +335,23 @@ class SplashAttentionKernel:
       return bs.block_q
     return self._auto_forward_tiling(head_dim, head_dim_v, **kw)[0]
 
-  def _call_block_sizes(self, head_dim: int, head_dim_v: int, itemsize: int, has_segments: bool) -> BlockSizes:
-    """`resolved_block_sizes` of a call, worked out once per class of calls."""
-    key = (self.requested_block_sizes, head_dim, head_dim_v, itemsize, has_segments)
+  def _call_block_sizes(self, head_dim: int, head_dim_v: int, itemsize: int, has_segments: bool,
+                        tiles: int | None) -> BlockSizes:
+    """`resolved_block_sizes` of a call, worked out once per class of calls: it depends on `tiles` only
+    through the bounds that `_auto_forward_tiling` compares it with."""
+    if tiles is not None:
+      tiles = next((n for n in cfg.FEW_TILES if tiles <= n), None)
+    key = (self.requested_block_sizes, head_dim, head_dim_v, itemsize, has_segments, tiles)
     bs = self._resolved.get(key)
     if bs is None:
       bs = self._resolved[key] = self.resolved_block_sizes(head_dim, head_dim_v, itemsize=itemsize,
-                                                           has_segments=has_segments)
+                                                           has_segments=has_segments, tiles=tiles)
     return bs
 
   def resolved_block_sizes(self, head_dim: int, head_dim_v: int, **kw) -> BlockSizes:
     bs = self.requested_block_sizes
+    if bs.block_kv is not None or bs.num_stages is not None:
+      kw["tiles"] = None  # a tiling of which a part is given keeps the shape it was given for
     if bs.block_q is None:
       bq, bkv, stages = self._auto_forward_tiling(head_dim, head_dim_v, **kw)
     else:
@@ -363,8 +388,13 @@ class SplashAttentionKernel:
       raise NotImplementedError(
           "interpret= selects the reference's CPU interpreter; this library"
           " only runs on an sm_100a GPU.")
+    # Calls that a backward pass follows keep a tiling that does not depend on how much is in the call, so
+    # that a (batch, head) unit has the same results to the bit in every call; the others may choose by it.
+    needs_grad = (not save_residuals and torch.is_grad_enabled()
+                  and any(isinstance(x, torch.Tensor) and x.requires_grad for x in (q, k, v)))
     bs = self._call_block_sizes(
-        q.shape[-1], v.shape[-1], q.element_size(), segment_ids is not None)
+        q.shape[-1], v.shape[-1], q.element_size(), segment_ids is not None,
+        None if needs_grad else math.prod(q.shape[:-1]) // cfg.TILE_ROWS)
     return _splash_attention(self, bs, q, k, v, segment_ids,
                              save_residuals=save_residuals)
 
@@ -406,7 +436,7 @@ def _splash_attention(kernel: SplashAttentionKernel, bs: BlockSizes, q, k, v,
     segment_ids = SegmentIds(_as_segment_tensor(seg_q, q.shape[0], q.device),
                              _as_segment_tensor(seg_kv, q.shape[0], q.device))
   if save_residuals:
-    out, lse = _forward(kernel, bs, q, k, v, segment_ids, save_residuals=True)
+    out, lse = _forward(kernel, bs, q, k, v, segment_ids, save_residuals=True, shared_tiles=True)
   else:
     seg_q = segment_ids.q if segment_ids is not None else None
     seg_kv = segment_ids.kv if segment_ids is not None else None
@@ -521,8 +551,10 @@ def _base_params(kernel: SplashAttentionKernel, q, k, v, segment_ids,
 
 
 def _forward(kernel: SplashAttentionKernel, bs: BlockSizes, q, k, v,
-             segment_ids, *, save_residuals: bool):
-  """Runs one forward kernel; returns (out, lse or None)."""
+             segment_ids, *, save_residuals: bool, shared_tiles: bool):
+  """Runs one forward kernel; returns (out, lse or None).  `shared_tiles`: several CTAs may take one
+  q tile where the tiles alone would leave SMs idle (results then depend on the number of tiles to
+  rounding)."""
   lib = _ffi.load()
   _poll_status(q.device)
   sched = kernel._fwd_schedule(bs, q.device)
@@ -538,8 +570,14 @@ def _forward(kernel: SplashAttentionKernel, bs: BlockSizes, q, k, v,
   p.block_q, p.block_kv, p.num_stages = bs.block_q, bs.block_kv, bs.num_stages
   with _on_device(q.device):
     stream = _raw_stream(q.device)
-    entry = lib.splash_fwd256 if bs.block_q == cfg.PINGPONG_ROWS else lib.splash_fwd128
-    _ffi.check(entry(ctypes.byref(p), stream), "splash attention forward")
+    nbytes = int(lib.splash_fwd_split_bytes(ctypes.byref(p))) if shared_tiles else 0
+    if nbytes > 0:
+      parts = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+      rc = lib.splash_fwd_split(ctypes.byref(p), parts.data_ptr(), nbytes, stream)
+    else:
+      entry = lib.splash_fwd256 if bs.block_q == cfg.PINGPONG_ROWS else lib.splash_fwd128
+      rc = entry(ctypes.byref(p), stream)
+    _ffi.check(rc, "splash attention forward")
   _maybe_check(q.device)
   return out, lse
 
@@ -662,7 +700,7 @@ class _SplashAttentionFn(torch.autograd.Function):
     segment_ids = None if seg_q is None else SegmentIds(seg_q, seg_kv)
     need_grad = any(ctx.needs_input_grad[:3])
     out, lse = _forward(kernel, bs, q, k, v, segment_ids,
-                        save_residuals=need_grad)
+                        save_residuals=need_grad, shared_tiles=not need_grad)
     if need_grad:
       ctx.save_for_backward(q, k, v, out, lse, *(() if seg_q is None else (seg_q, seg_kv)))
       ctx.kernel, ctx.bs = kernel, bs
