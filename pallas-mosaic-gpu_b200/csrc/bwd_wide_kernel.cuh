@@ -600,7 +600,9 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             tc_fence_before();
             mbar_arrive(SPLASH_WBAR(s_free, 0));
           }
-          uint32_t ppk[32];
+          // P^T leaves in halves where its columns are this thread's own, which keeps the registers of the
+          // row, the packed values and the step's bookkeeping within the budget.
+          uint32_t ppk[L::kRoomy ? 32 : 16];
           const uint32_t vec = lse_u32 + slot * L::kVecBytes + col0 * 4;
           // One straight-line body per (soft-cap, masking) combination; the step picks one.
           // Masked entries and rows that saw no key (lse == mask_value) get an exponent of
@@ -645,10 +647,13 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                   if (!((vis[i >> 5] >> ((i + 1) & 31)) & 1u)) x.y = -INFINITY;
                 }
                 const float2 p = make_float2(ex2_approx(x.x), ex2_approx(x.y));
-                ppk[g * 2 + e] = pack2<BF16>(p.x, p.y);
+                ppk[(L::kRoomy ? g : g % 8) * 2 + e] = pack2<BF16>(p.x, p.y);
                 const float2 f = kCap ? mul2(p, keep) : p;
                 pf[i] = f.x;
                 pf[i + 1] = f.y;
+              }
+              if constexpr (!L::kRoomy) {
+                if (g % 8 == 7) tmem_st16(tmem_row + L::kColP + w * L::kPHalf + (g / 8) * 16, ppk);
               }
             }
           };
@@ -666,7 +671,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             tc_fence_after();
           }
           // Packed P^T; without columns of its own, over the first half of those this thread just read.
-          tmem_st32(tmem_row + L::kColP + w * L::kPHalf, ppk);
+          if constexpr (L::kRoomy) tmem_st32(tmem_row + L::kColP + w * L::kPHalf, ppk);
           tmem_wait_st();
           tc_fence_before();
           mbar_arrive(SPLASH_WBAR(p_ready, 0));
