@@ -111,8 +111,9 @@ struct FwdLayout {
   static_assert(kTmemCols <= 512 / kCtasPerSm, "tensor memory has 512 columns per SM");
   static constexpr int kSoftmaxGroups = NT * AW;
   static constexpr int kThreads = (kSoftmaxGroups + 1) * 128;
-  // Row maxima shared by the alternating warpgroups, and their partial row sums.
-  static constexpr int kShareBytes = AW > 1 ? 3 * kTile * 4 : 0;
+  // Row maxima shared by the alternating warpgroups.  (Their partial row sums, posted in the epilogue, go
+  // into the K ring, which is dead by then: a ring depth that fits one group fits two.)
+  static constexpr int kShareBytes = AW > 1 ? kTile * 4 : 0;
   static constexpr bool kOStageInQ = (NT == 2) || (DV <= D);
   // Register split between the warpgroups when there are two softmax warpgroups
   // (multiples of 8).  One CTA per SM starts with 168 registers a thread: 384 * 168 = 256 * 216 +
@@ -182,7 +183,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const uint32_t mask_u32 = v_u32 + stages * L::kVStage;
   const uint32_t seg_u32 = mask_u32 + (has_dense ? stages * L::kMaskStage : 0);
   const uint32_t bars_u32 = seg_u32 + (has_seg ? stages * L::kSegStage : 0);
-  const uint32_t share_u32 = bars_u32 + 1024;  // [row maxima | partial sums of group 0 | of group 1]
+  const uint32_t share_u32 = bars_u32 + 1024;  // row maxima
   const uint32_t abort_u32 = bars_u32 + static_cast<uint32_t>(offsetof(FwdBarriers, abort_flag));
   const uint32_t tmem_slot_u32 = bars_u32 + static_cast<uint32_t>(offsetof(FwdBarriers, tmem_base));
   const uint32_t dead_u32 = bars_u32 + static_cast<uint32_t>(offsetof(FwdBarriers, dead));
@@ -485,7 +486,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const uint32_t tmem_row = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
     const uint32_t o_tmem = tmem_row + L::kOCol + t * DV;
     const uint32_t m_sh = share_u32 + row * 4;                    // the row's maximum after the latest step
-    const uint32_t l_sh = share_u32 + (1 + grp) * kTile * 4 + row * 4;  // this group's partial row sum
+    const uint32_t l_sh = k_u32 + grp * kTile * 4 + row * 4;      // this group's partial row sum (epilogue)
     constexpr int kEpiCols = DV / AW;                             // columns of O per thread in the epilogue
     const int epi_col0 = (AW == 2) ? grp * kEpiCols : 0;
 
@@ -732,7 +733,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           mbar_arrive(SPLASH_BAR(fin, 0));
           alive = warp_wait(SPLASH_BAR(fin, 0), 0, ctx, kSiteSmxFin, n);
         }
-        if (alive) l_tot = l_run + __uint_as_float(lds32(share_u32 + (1 + (grp ^ 1)) * kTile * 4 + row * 4));
+        if (alive) l_tot = l_run + __uint_as_float(lds32(k_u32 + (grp ^ 1) * kTile * 4 + row * 4));
       }
       if (SPLIT && alive) {
         tc_fence_after();

@@ -41,3 +41,10 @@ def test_gpu_few_steps(d, kv):
   sa.check_device_status()
   ref, ref_lse = oracle.attention_forward(np.ones((1, 128, kv), bool), q, k, v)
   assert_forward_close(out, lse, ref, ref_lse, torch.bfloat16)
+
+
+def test_gpu_deepest_ring_that_one_group_had(monkeypatch):
+  """head_dim 128, head_dim_v 64 with eight stages fills shared memory to 512 bytes: the library takes it
+  (this package's own budget, the reference's formula, asks for more than the kernel uses)."""
+  monkeypatch.setattr(sa.config, "SMEM_BYTES", 1 << 20)
+  _check("causal", s=1024, d=128, dv=64, block_sizes=sa.BlockSizes(block_q=128, block_kv=64, num_stages=8))
