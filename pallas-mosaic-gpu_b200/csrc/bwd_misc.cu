@@ -8,6 +8,7 @@
 #include <cuda_fp16.h>
 
 #include "dispatch.h"
+#include "fold_weights.cuh"
 #include "host_common.cuh"
 #include "ptx.cuh"
 
@@ -23,27 +24,30 @@ __device__ __forceinline__ float2 unpack2(uint32_t w) {
   }
 }
 
-// Splits -x into three 16-bit floats whose sum is -x to f32 precision, as the eight 16-bit
-// values {hi, mid, lo, 0, 0, 0, 0, 0} per row that the 128-row fused backward (head_dim 64)
-// multiplies by {1, 1, 1, 0, ...} in one extra K = 16 slice of its score products.  Rows whose
-// lse is mask_value (they saw no key) get a large negative value instead, which makes their P zero.
+// Splits -x into 16-bit floats whose weighted sum is -x: the eight values per row that the 128-row fused
+// backward (head_dim 64) multiplies by FoldWeights in one extra K = 16 slice of its score products.
+// bf16 has the range of f32, so three parts of weight 1 hold all 24 bits.  f16 has not: its four parts are
+// weighted by powers of two, which takes |x| to 2.1e9 (parts of weight 1 end at 65504, and a larger part is an
+// infinity that turns every dP^T it is added to into NaN) and leaves at most max(2^-24 |x|, 2^-39).
+// Rows whose lse is mask_value (they saw no key) get a large negative value instead, which makes their P zero.
 template <bool BF16>
-__device__ __forceinline__ uint4 split3_neg(float x, bool sentinel) {
-  float v = sentinel ? (BF16 ? -1.0e30f : -60000.f) : -x;
-  uint32_t h[3];
+__device__ __forceinline__ uint4 split_neg(float x, bool sentinel) {
+  float v = sentinel ? (BF16 ? -1.0e30f : -2.0e9f) : -x;
+  uint32_t h[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < FoldWeights<BF16>::kParts; ++i) {
     if constexpr (BF16) {
       const __nv_bfloat16 b = __float2bfloat16_rn(v);
       h[i] = *reinterpret_cast<const uint16_t*>(&b);
       v -= __bfloat162float(b);
     } else {
-      const __half b = __float2half_rn(v);
+      const float w = FoldWeights<BF16>::weight(i);  // a power of two: scaling by it is exact
+      const __half b = __float2half_rn(v * (1.f / w));
       h[i] = *reinterpret_cast<const uint16_t*>(&b);
-      v -= __half2float(b);
+      v = fmaf(-w, __half2float(b), v);
     }
   }
-  return make_uint4(h[0] | (h[1] << 16), h[2], 0u, 0u);
+  return make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), 0u, 0u);
 }
 
 // delta = rowsum(dO * O), LPR lanes per row (as many as the row has 16-byte chunks, so that every lane
@@ -111,10 +115,10 @@ __global__ void __launch_bounds__(256) delta_kernel(const uint4* __restrict__ o,
     if (row < rows) {
       if (sub == 0) {
         delta[row] = v;
-        if (fold.aux_lse) fold.aux_delta[row] = split3_neg<BF16>(v, false);
+        if (fold.aux_lse) fold.aux_delta[row] = split_neg<BF16>(v, false);
       } else if (sub == 1 && fold.aux_lse) {
         const float l = fold.lse[row];
-        fold.aux_lse[row] = split3_neg<BF16>(l, l == fold.mask_value);
+        fold.aux_lse[row] = split_neg<BF16>(l, l == fold.mask_value);
       }
     }
   }
@@ -188,8 +192,8 @@ __global__ void __launch_bounds__(256) fold_operands_kernel(const float* __restr
   const long long r = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (r >= rows) return;
   const float l = lse[r];
-  aux_lse[r] = split3_neg<BF16>(l, l == mask_value);
-  aux_delta[r] = split3_neg<BF16>(delta[r], false);
+  aux_lse[r] = split_neg<BF16>(l, l == mask_value);
+  aux_delta[r] = split_neg<BF16>(delta[r], false);
 }
 
 int launch_fold_operands(const float* lse, const float* delta, void* aux_lse, void* aux_delta, long long rows,

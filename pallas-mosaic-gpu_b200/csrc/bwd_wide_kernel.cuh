@@ -50,6 +50,7 @@
 #include <type_traits>
 
 #include "bwd_col_kernel.cuh"  // BwdArgs, ColSteps, math constants
+#include "fold_weights.cuh"
 #include "ptx.cuh"
 
 // Timeline marks for debugging builds; empty in the product.
@@ -93,14 +94,14 @@ struct WideLayout {
   static constexpr int kOffLse = kOffDqStage + 4 * kDqBufs * kDqBoxBytes, kOffDelta = kOffLse + kSlots * kVecBytes;
   // Folded operands (head_dim 64, where shared memory has the room): -lse and -delta are subtracted
   // inside the S^T and dP^T products by one extra K = 16 slice each.  Per q row eight 16-bit values
-  // {hi, mid, lo, 0, ...} whose sum is -lse (or -delta) to f32 precision -- the first 8 x 8 core
-  // matrices of an unswizzled K-major tile -- against {1, 1, 1, 0, ...} per kv row; the second half of
+  // {hi, mid, lo, ...} whose sum under FoldWeights is -lse (or -delta) -- the first 8 x 8 core
+  // matrices of an unswizzled K-major tile -- against the weights per kv row; the second half of
   // K is a shared block of zeros.
   static constexpr bool kFold = D == 64;
   static constexpr int kAuxTile = BC * 16;
   static constexpr int kOffAux = kOffDelta + kSlots * kVecBytes;                  // per Q slot: [-lse tile | -delta tile]
-  static constexpr int kOffOnes = kOffAux + (kFold ? kSlots * 2 * kAuxTile : 0);
-  static constexpr int kOffZeros = kOffOnes + (kFold ? kAuxTile : 0);
+  static constexpr int kOffWeights = kOffAux + (kFold ? kSlots * 2 * kAuxTile : 0);
+  static constexpr int kOffZeros = kOffWeights + (kFold ? kAuxTile : 0);
   static constexpr int kOffBars = kOffZeros + (kFold ? kAuxTile : 0);
   static constexpr int kBarBytes = 256;
   static constexpr int kListSteps = 256;  // capacity of the list of block steps that survive segment skipping
@@ -175,7 +176,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   const uint32_t lse_u32 = base_u32 + L::kOffLse;
   const uint32_t delta_u32 = base_u32 + L::kOffDelta;
   const uint32_t aux_u32 = base_u32 + L::kOffAux;
-  const uint32_t ones_u32 = base_u32 + L::kOffOnes;
+  const uint32_t weights_u32 = base_u32 + L::kOffWeights;
   const uint32_t zeros_u32 = base_u32 + L::kOffZeros;
   // With soft-capping lse has to be subtracted after the cap, so only delta is folded then.
   const bool fold_lse = L::kFold && !(soft_cap > 0.f);
@@ -250,10 +251,9 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   }
   if constexpr (L::kFold) {
     if (threadIdx.x >= 64 && threadIdx.x < 64 + 256) {
-      // 128 rows of {1, 1, 1, 0, 0, 0, 0, 0}, and 2 KB of zeros.
+      // 128 rows of the parts' weights, and 2 KB of zeros.
       const uint32_t i = threadIdx.x - 64;
-      const uint32_t one = BF16 ? 0x3f80u : 0x3c00u;
-      if (i < 128) sts128(ones_u32 + i * 16, make_uint4(one | (one << 16), one, 0u, 0u));
+      if (i < 128) sts128(weights_u32 + i * 16, make_uint4(FoldWeights<BF16>::kLo, FoldWeights<BF16>::kHi, 0u, 0u));
       else sts128(zeros_u32 + (i - 128) * 16, make_uint4(0u, 0u, 0u, 0u));
       fence_proxy_async_smem();
     }
@@ -341,10 +341,10 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           umma_ss2_w(tmem + d_col, a_lo + o, kDescHi, b_lo + o, kDescHi, kIdescScore, kk > 0);
         }
       };
-      // One more K = 16 slice: D[kv, q] += sum_k ones[kv, k] * aux[q, k] = -lse[q] (or -delta[q]);
+      // One more K = 16 slice: D[kv, q] += sum_k weights[kv, k] * aux[q, k] = -lse[q] (or -delta[q]);
       // both operands unswizzled K-major, the second half of K read from the block of zeros.
       auto issue_fold = [&](uint32_t d_col, uint32_t b_tile) {
-        umma_ss2_w(tmem + d_col, desc_lo_plain(ones_u32, zeros_u32 - ones_u32), desc_hi_plain(128),
+        umma_ss2_w(tmem + d_col, desc_lo_plain(weights_u32, zeros_u32 - weights_u32), desc_hi_plain(128),
                    desc_lo_plain(b_tile, zeros_u32 - b_tile), desc_hi_plain(128), kIdescScore, 1u);
       };
       // A = packed 16-bit values the elementwise warps left in tensor memory: q columns

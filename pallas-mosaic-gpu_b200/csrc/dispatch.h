@@ -39,7 +39,7 @@ int launch_delta(const void* o, const void* d_out, float* delta, long long rows,
                  void* aux_lse = nullptr, void* aux_delta = nullptr, float mask_value = 0.f);
 int launch_dq_cast(const float* acc, void* dq, long long batch_heads, int head_dim, int q_len, int dtype,
                    cudaStream_t stream);
-// -lse and -delta of every q row as three 16-bit parts each (16 bytes per row and array): the
+// -lse and -delta of every q row as 16-bit parts (FoldWeights) (16 bytes per row and array): the
 // operands of the slice that the 128-row fused backward adds to its score products at head_dim 64.
 int launch_fold_operands(const float* lse, const float* delta, void* aux_lse, void* aux_delta, long long rows,
                          float mask_value, int dtype, cudaStream_t stream);

@@ -2,9 +2,14 @@
 (read per thread, straight from memory), the shortest and odd step counts of its rings, per-head
 masks and grouped heads; against the CPU oracle with the bars of test_gpu_backward.py."""
 
+import numpy as np
 import pytest
 import torch
 
+import splash_attention_mgpu as sa
+from oracle import dense_attention as oracle
+
+from common import build_mask, inputs
 from test_gpu_backward import _check_grads, _id
 
 pytestmark = pytest.mark.gpu
@@ -24,3 +29,28 @@ CASES = [
 def test_gpu_wide_backward(kwargs):
   kwargs = dict(kwargs)
   _check_grads(kwargs.pop("mask_name"), scaled=True, **kwargs)
+
+
+@pytest.mark.parametrize("mask_name,cap,h,kvh", [("dense", None, 2, 2), ("causal", None, 2, 2), ("full", 20.0, 4, 2)])
+def test_gpu_f16_delta_beyond_the_range_of_f16(mask_name, cap, h, kvh):
+  """Loss-scaled f16 gradients: rows whose delta = dO . O is above 65504 while every operand and gradient is
+  finite.  delta comes from the output rounded to f16 (2^-11 of 200 a value, eight values' worth in the root of the
+  64 terms), dP - delta from values 20 wide: that alone is 200 / 2^11 / sqrt(3) / 20 = 0.3 % of a score's gradient."""
+  s, d = 384, 64
+  mask, dense = build_mask(mask_name, s, h, False)
+  kernel = sa.make_splash_mha(mask, attn_logits_soft_cap=cap)
+  q, k, v = inputs(1, h, kvh, s, d, d, torch.float16, False, seed=3, device="cuda:0", scale=d ** -0.5)
+  v = 200 + 20 * v
+  g = torch.Generator().manual_seed(5)
+  d_out = (40 + 8 * torch.randn(q.shape, generator=g)).to(torch.float16).to("cuda:0")
+  qg, kg, vg = (x.clone().requires_grad_(True) for x in (q, k, v))
+  out = kernel(qg, kg, vg)
+  got = torch.autograd.grad(out, (qg, kg, vg), d_out)
+  sa.check_device_status()
+  assert float((d_out.float() * out.detach().float()).sum(-1).abs().min()) > 65504
+  want = oracle.attention_backward(dense, q, k, v, d_out, attn_logits_soft_cap=cap)
+  for name, x, r in zip("qkv", got, want):
+    x = x.float().cpu().numpy()
+    assert np.isfinite(x).all(), name
+    assert np.abs(x - r).max() / np.abs(r).max() < 2e-2, name
+    assert np.abs(x - r).mean() / np.abs(r).mean() <= 1e-2, name
