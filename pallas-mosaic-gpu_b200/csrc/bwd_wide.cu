@@ -33,8 +33,8 @@ static int launch_bwd_wide_typed(const SplashParams& p, cudaStream_t stream) {
   a.stages = L::kSlots;
   a.aux_lse = fold_operand_lse(p);  // filled by the caller
   a.aux_delta = fold_operand_delta(p);
-  // Segment skipping when the CTA's list of block steps fits the room set aside for it.
-  const bool skipping = seg && p.seg_ranges != nullptr && (p.heads / p.kv_heads) * p.max_steps <= L::kListSteps;
+  // Segment skipping when what is left of the CTA's block steps fits the room set aside for it.
+  const bool skipping = seg && p.seg_ranges != nullptr && L::steps_fit(p.mask_heads > 1 ? p.heads / p.kv_heads : 1, p.max_steps);
   a.seg_q_ranges = skipping ? seg_q_ranges(p) : nullptr;
   a.seg_kv_ranges = skipping ? seg_kv_ranges(p) : nullptr;
   const bool plain = p.soft_cap == 0.f && !seg;

@@ -104,9 +104,21 @@ struct WideLayout {
   static constexpr int kOffZeros = kOffWeights + (kFold ? kAuxTile : 0);
   static constexpr int kOffBars = kOffZeros + (kFold ? kAuxTile : 0);
   static constexpr int kBarBytes = 256;
-  static constexpr int kListSteps = 256;  // capacity of the list of block steps that survive segment skipping
-  static constexpr int kOffList = kOffBars + kBarBytes;
-  static constexpr int kSmemBytes = kOffList + kListSteps * 2;
+  // Segment skipping: which block steps are left, in rows of one head (one row where all heads share a mask): a list of
+  // 16-bit entries at head_dim 64; at head_dim 128, where shared memory has 1 KB left, two bits a scheduled step, which
+  // hold 3071 steps of a row.  (A list of all heads of the group ended at 256 steps there, which 8 q heads a KV head
+  // reach at 4096 tokens; 16 q and 2 KV heads, 8192 tokens, an array mask and packed documents, backward call:
+  // 1507 -> 662 us, at head_dim 64 1150 -> 491; calls of fewer steps 0 at head_dim 64, 0 to +4 % at 128.)
+  static constexpr bool kStepBits = D == 128;
+  static constexpr int kStepBytes = kStepBits ? 768 : 20480;
+  static constexpr int kOffSteps = kOffBars + kBarBytes;
+  static constexpr int kSmemBytes = kOffSteps + kStepBytes;
+  __host__ __device__ static constexpr int step_row_bytes(int max_steps) {
+    return kStepBits ? (max_steps / 32 + 1) * 4 : (max_steps + 1) * 2;
+  }
+  __host__ static constexpr bool steps_fit(int rows, int max_steps) {
+    return max_steps < 0x7fff && static_cast<long long>(rows) * step_row_bytes(max_steps) <= (kStepBits ? kStepBytes / 2 : kStepBytes);
+  }
   static_assert(kSmemBytes <= 227 * 1024, "shared memory per CTA");
   // Tensor memory columns.
   static constexpr int kColS = 0, kColDp = 128, kColDk = 256, kColDv = 256 + D;
@@ -126,6 +138,96 @@ struct Ring {
   uint32_t phase = 0;
   __device__ __forceinline__ void next() {
     if (++slot == N) { slot = 0; phase ^= 1; }
+  }
+};
+
+// Enumerates the block steps of one CTA, (q head of the group, visited q block) pairs in that order; with segment
+// skipping only those left in a row of bits or a list (L::kStepBits).  Where all heads share one mask the q heads of a
+// group visit the same blocks, and as ids do not depend on the head, one row serves them all.
+template <class L>
+struct WideSteps {
+  const BwdArgs* a;
+  int kj, head0, group;
+  bool skipping;
+  int count, e;      // steps to walk, position in that sequence
+  int g, i;          // head; step inside the head, with a list the entry of the step
+  int n, base;       // scheduled steps of head g and, where nothing is skipped, before it
+  uint32_t entry;    // list: step inside the head, kSegUniformBit
+  uint32_t row_u32;  // row of head g
+
+  __device__ __forceinline__ int mask_head(int gg) const { return a->mask_heads > 1 ? head0 + gg : 0; }
+  __device__ __forceinline__ int steps_of(int gg) const { return a->num_steps[mask_head(gg) * a->kv_blocks + kj]; }
+  __device__ __forceinline__ int list_off(int gg) const { return (mask_head(gg) * a->kv_blocks + kj) * a->max_steps; }
+  __device__ __forceinline__ int row_bytes() const { return a->mask_heads > 1 ? L::step_row_bytes(a->max_steps) : 0; }
+  __device__ __forceinline__ void bind(const BwdArgs* args, int kj_, int head0_, int group_) {
+    a = args; kj = kj_; head0 = head0_; group = group_;
+  }
+  // Scheduled block steps of the CTA, before any skipping.
+  __device__ __forceinline__ int scheduled() const {
+    int t = 0;
+    for (int gg = 0; gg < group; ++gg) t += steps_of(gg);
+    return t;
+  }
+  // One warp: writes the rows; `classify` gets an offset into the step lists.  Returns the steps left in the CTA.
+  template <typename F>
+  __device__ __forceinline__ int build(uint32_t steps_u32, int lane, F classify) const {
+    const int rows = a->mask_heads > 1 ? group : 1;
+    int kept = 0;
+    for (int gg = 0; gg < rows; ++gg) {
+      const uint32_t row = steps_u32 + gg * row_bytes();
+      auto of_step = [&](int f) { return classify(list_off(gg) + f); };
+      if constexpr (L::kStepBits) {
+        kept += build_step_bits(row, row + L::kStepBytes / 2, steps_of(gg), lane, of_step);
+      } else {
+        const int in_row = build_step_list(row, steps_of(gg), lane, of_step);
+        if (lane == 0) sts16(row + 2u * in_row, kSegListEnd);
+        kept += in_row;
+      }
+    }
+    return rows == 1 ? kept * group : kept;
+  }
+  // To step e of the CTA: the first one that is left at position f of the row of head g or behind it.
+  __device__ __forceinline__ void seek(int f) {
+    if (!skipping) {
+      while (e >= base + n) { base += n; ++g; n = steps_of(g); }
+      i = e - base;
+      return;
+    }
+    if constexpr (L::kStepBits) {
+      while ((f = next_step_bit(row_u32, f)) == n) {
+        ++g;
+        row_u32 += row_bytes();
+        n = steps_of(g);
+        f = 0;
+      }
+    } else {
+      while ((entry = lds16(row_u32 + 2u * f)) == kSegListEnd) {
+        ++g;
+        row_u32 += row_bytes();
+        f = 0;
+      }
+    }
+    i = f;
+  }
+  __device__ __forceinline__ void start(uint32_t steps_u32, bool with_rows, int count_) {
+    row_u32 = steps_u32; skipping = with_rows; count = count_;
+    e = 0; g = 0; i = 0; entry = 0; base = 0;
+    n = steps_of(0);
+    if (count > 0) seek(0);
+  }
+  __device__ __forceinline__ bool valid() const { return e < count; }
+  __device__ __forceinline__ void next() {
+    if (++e < count) seek(i + 1);
+  }
+  __device__ __forceinline__ int head() const { return head0 + g; }
+  __device__ __forceinline__ int off() const {
+    return list_off(g) + (skipping && !L::kStepBits ? static_cast<int>(entry & ~kSegUniformBit) : i);
+  }
+  // Both sides of the block carry one and the same segment id: nothing to compare.
+  __device__ __forceinline__ bool uniform() const {
+    if (!skipping) return false;
+    if (!L::kStepBits) return entry & kSegUniformBit;
+    return (lds32(row_u32 + L::kStepBytes / 2 + 4u * (i >> 5)) >> (i & 31)) & 1u;
   }
 };
 
@@ -185,8 +287,8 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   const uint32_t dead_u32 = bars_u32 + static_cast<uint32_t>(offsetof(WideBarriers, dead));
   const uint32_t tmem_slot_u32 = bars_u32 + static_cast<uint32_t>(offsetof(WideBarriers, tmem_base));
   const uint32_t neff_u32 = bars_u32 + static_cast<uint32_t>(offsetof(WideBarriers, n_eff));
-  const uint32_t list_u32 = base_u32 + L::kOffList;
-  const bool has_list = has_seg && a.seg_q_ranges != nullptr;
+  const uint32_t steps_u32 = base_u32 + L::kOffSteps;
+  const bool skipping = has_seg && a.seg_q_ranges != nullptr;
 
   const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
@@ -202,7 +304,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   const int kj = a.block_order[mh0 * a.kv_blocks + order_idx];
   const int kv_row0 = (b * a.kv_heads + kvh) * a.kv_len + kj * kRows;  // row in the [B*KVH*Skv, D] view
 
-  ColSteps<1> it;
+  WideSteps<L> it;
   it.bind(&a, kj, head0, group);
   const int scheduled = it.scheduled();
 
@@ -238,14 +340,13 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   } else if (warp == kProducerWarp0 + 1) {
     tmem_alloc(tmem_slot_u32, L::kTmemCols);
     tmem_relinquish();
-  } else if (warp == 1 && has_list) {
+  } else if (warp == 1 && skipping) {
     // Block steps whose q and kv segment-id ranges can meet; the others are left out by every role.
     const int2* qt = a.seg_q_ranges + static_cast<size_t>(b) * (a.q_len / kSegChunk);
     const int2* kt = a.seg_kv_ranges + static_cast<size_t>(b) * (a.kv_len / kSegChunk);
     const SegRange kr = seg_range(kt, kj * (kRows / kSegChunk), kRows / kSegChunk);
-    const int kept = build_step_list(list_u32, scheduled, lane, [&](int f) {
-      const int qblk = a.block_list[it.off_of_flat(f)];
-      return seg_classify(seg_range(qt, qblk * (128 / kSegChunk), 128 / kSegChunk), kr);
+    const int kept = it.build(steps_u32, lane, [&](int off) {
+      return seg_classify(seg_range(qt, a.block_list[off] * (128 / kSegChunk), 128 / kSegChunk), kr);
     });
     if (lane == 0) sts32(neff_u32, static_cast<uint32_t>(kept));
   }
@@ -263,8 +364,8 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   tc_fence_after();
   const uint32_t tmem = lds32(tmem_slot_u32);
   const WaitCtx ctx{abort_u32};
-  it.start(list_u32, has_list, has_list ? static_cast<int>(lds32(neff_u32)) : scheduled);
-  const int total = it.total();
+  const int total = skipping ? static_cast<int>(lds32(neff_u32)) : scheduled;
+  it.start(steps_u32, skipping, total);
   if (lds32(dead_u32)) {
     if (warp == kProducerWarp0 + 1) {
       __syncwarp();

@@ -11,7 +11,8 @@
 // Before its first barrier one warp of a CTA walks the CTA's scheduled steps, classifies
 // them and writes the steps that remain to a list in shared memory (16-bit entries: step
 // index, top bit set when the ids are uniform); every role then iterates that list, so
-// all roles agree on the steps without any of them re-deriving the decision.
+// all roles agree on the steps without any of them re-deriving the decision.  Where
+// there is no room for a list two bits per scheduled step (kept, uniform) take its place.
 #pragma once
 
 #include "ptx.cuh"
@@ -21,6 +22,7 @@ namespace splash {
 constexpr int kSegChunk = 64;  // positions per recorded (min, max) pair
 enum SegKind : int { kSegSkip = 0, kSegMixed = 1, kSegUniform = 2 };
 constexpr uint32_t kSegUniformBit = 0x8000u;
+constexpr uint32_t kSegListEnd = 0xffffu;  // behind the last entry, where a walk over a list has to notice its end
 
 struct SegRange {
   int lo, hi;
@@ -68,6 +70,36 @@ __device__ __forceinline__ int build_step_list(uint32_t list_u32, int n, int lan
     count += __popc(keep);
   }
   return count;
+}
+
+// The same decision as two rows of bits, kept steps at `kept_u32` and uniform ones at `uniform_u32`.  Bit n of the
+// first, behind the last step, is set as well: a walk from set bit to set bit ends there.  Returns the number of kept
+// steps.
+template <typename F>
+__device__ __forceinline__ int build_step_bits(uint32_t kept_u32, uint32_t uniform_u32, int n, int lane, F classify) {
+  int count = 0;
+  for (int base = 0; base <= n; base += 32) {
+    const int i = base + lane;
+    const int c = i < n ? classify(i) : static_cast<int>(kSegSkip);
+    const uint32_t keep = __ballot_sync(0xffffffffu, c != kSegSkip);
+    const uint32_t same = __ballot_sync(0xffffffffu, c == kSegUniform);
+    if (lane == 0) {
+      sts32(kept_u32 + (base >> 3), n - base < 32 ? keep | (1u << (n - base)) : keep);
+      sts32(uniform_u32 + (base >> 3), same);
+    }
+    count += __popc(keep);
+  }
+  return count;
+}
+
+// First set bit at or after bit f of a row (there is one).
+__device__ __forceinline__ int next_step_bit(uint32_t row_u32, int f) {
+  uint32_t w = lds32(row_u32 + 4u * (f >> 5)) & (0xffffffffu << (f & 31));
+  while (w == 0) {
+    f = (f | 31) + 1;
+    w = lds32(row_u32 + 4u * (f >> 5));
+  }
+  return (f & ~31) + __ffs(w) - 1;
 }
 
 }  // namespace splash

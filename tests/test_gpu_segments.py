@@ -117,3 +117,40 @@ def test_q_blocks_whose_every_step_is_skipped(d, bs, fused, monkeypatch):
   # (reference tools/fuzz.py:116-124), so gradients are compared where only live rows contribute.
   got_dq = qg.grad[0, :, live].float().cpu().numpy()
   assert np.abs(got_dq - ref[0][0, :, live]).max() / np.abs(ref[0][0, :, live]).max() < 2e-2
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("mask_name,h,kvh,s", [
+    ("array", 8, 1, 4352),    # 34 blocks x 8 heads of the group: 272 scheduled steps a CTA
+    ("array", 2, 2, 4224),    # one head a CTA, 33 steps: the walk ends in the second word of its bits
+    ("causal", 8, 1, 4352),
+    ("per_head", 8, 1, 4352),  # a row of bits per head
+    ("per_head", 6, 2, 1024),
+])
+def test_backward_leaves_out_blocks_at_any_number_of_steps(mask_name, h, kvh, s, d):
+  """Documents of 256 tokens with NaN in one document's values: 0 * NaN would carry it into the dQ and dK of every
+  document whose blocks are computed against it, so finite gradients say that those blocks were left out."""
+  dense = np.tril(np.ones((s, s), bool)) & (np.random.default_rng(0).random((s, s), dtype=np.float32) > 0.3)
+  dense |= np.eye(s, dtype=bool)
+  causal = sa.CausalMask((s, s))
+  mask = {"array": lambda: sa.NumpyMask(dense), "causal": lambda: causal,
+          "per_head": lambda: sa.MultiHeadMask([causal if i % 2 else sa.ChunkedCausalMask((s, s), chunk_size=640)
+                                                for i in range(h)])}[mask_name]()
+  kernel = sa.make_splash_mha(mask)
+  q, k, v = inputs(1, h, kvh, s, d, d, torch.bfloat16, False, seed=4, device=DEV, scale=d ** -0.5)
+  do = torch.randn(q.shape, generator=torch.Generator().manual_seed(8)).to(torch.bfloat16).to(DEV)
+  ids = torch.arange(s, device=DEV, dtype=torch.int32) // 256
+  bad = ids == 3
+  poisoned = v.clone()
+  poisoned[:, :, bad] = float("nan")
+
+  def grads(values):
+    x = [t.clone().requires_grad_(True) for t in (q, k, values)]
+    return torch.autograd.grad(kernel(*x, sa.SegmentIds(ids, ids)), x, do)
+
+  want, got = grads(v), grads(poisoned)
+  sa.check_device_status()
+  for name, a, b in zip(("dq", "dk", "dv"), got, want):
+    a, b = a[:, :, ~bad].float(), b[:, :, ~bad].float()
+    assert bool(torch.isfinite(a).all()), name
+    np.testing.assert_allclose(a.cpu().numpy(), b.cpu().numpy(), atol=2e-3, rtol=2e-2, err_msg=name)
