@@ -390,13 +390,14 @@ class SplashAttentionKernel:
           " only runs on an sm_100a GPU.")
     # Calls that a backward pass follows keep a tiling that does not depend on how much is in the call, so
     # that a (batch, head) unit has the same results to the bit in every call; the others may choose by it.
+    # Decided here alone: inside an autograd function needs_input_grad stays set under no_grad.
     needs_grad = (not save_residuals and torch.is_grad_enabled()
                   and any(isinstance(x, torch.Tensor) and x.requires_grad for x in (q, k, v)))
     bs = self._call_block_sizes(
         q.shape[-1], v.shape[-1], q.element_size(), segment_ids is not None,
         None if needs_grad else math.prod(q.shape[:-1]) // cfg.TILE_ROWS)
     return _splash_attention(self, bs, q, k, v, segment_ids,
-                             save_residuals=save_residuals)
+                             save_residuals=save_residuals, needs_grad=needs_grad)
 
 
 # ---------------------------------------------------------------------------
@@ -414,7 +415,7 @@ def _as_segment_tensor(x, batch, device):
 
 
 def _splash_attention(kernel: SplashAttentionKernel, bs: BlockSizes, q, k, v,
-                      segment_ids, *, save_residuals: bool):
+                      segment_ids, *, save_residuals: bool, needs_grad: bool):
   if not (isinstance(q, torch.Tensor) and isinstance(k, torch.Tensor)
           and isinstance(v, torch.Tensor)):
     raise TypeError("q, k, v must be torch tensors")
@@ -440,7 +441,7 @@ def _splash_attention(kernel: SplashAttentionKernel, bs: BlockSizes, q, k, v,
   else:
     seg_q = segment_ids.q if segment_ids is not None else None
     seg_kv = segment_ids.kv if segment_ids is not None else None
-    out = _SplashAttentionFn.apply(q, k, v, seg_q, seg_kv, kernel, bs)
+    out = _SplashAttentionFn.apply(q, k, v, seg_q, seg_kv, kernel, bs, needs_grad)
     lse = None
   if not batched:
     out = out[0]
@@ -696,12 +697,11 @@ class _SplashAttentionFn(torch.autograd.Function):
   """Custom VJP: forward saves (q, k, v, out, lse); backward runs the dQ/dK/dV kernels."""
 
   @staticmethod
-  def forward(ctx, q, k, v, seg_q, seg_kv, kernel, bs):
+  def forward(ctx, q, k, v, seg_q, seg_kv, kernel, bs, needs_grad):
     segment_ids = None if seg_q is None else SegmentIds(seg_q, seg_kv)
-    need_grad = any(ctx.needs_input_grad[:3])
     out, lse = _forward(kernel, bs, q, k, v, segment_ids,
-                        save_residuals=need_grad, shared_tiles=not need_grad)
-    if need_grad:
+                        save_residuals=needs_grad, shared_tiles=not needs_grad)
+    if needs_grad:
       ctx.save_for_backward(q, k, v, out, lse, *(() if seg_q is None else (seg_q, seg_kv)))
       ctx.kernel, ctx.bs = kernel, bs
     return out
@@ -713,7 +713,7 @@ class _SplashAttentionFn(torch.autograd.Function):
     segment_ids = SegmentIds(saved[5], saved[6]) if len(saved) > 5 else None
     dq, dk, dv = _backward(ctx.kernel, ctx.bs, q.contiguous(), k.contiguous(),
                            v.contiguous(), segment_ids, out, lse, d_out)
-    return dq, dk, dv, None, None, None, None
+    return dq, dk, dv, None, None, None, None, None
 
 
 # ---------------------------------------------------------------------------

@@ -127,3 +127,18 @@ def test_gpu_calls_with_a_backward_do_not_share():
   whole, alone = run(q, k, v), run(q[1:, 2:3], k[1:, 2:3], v[1:, 2:3])
   for a, b in zip(whole, alone):
     assert torch.equal(a[1, 2], b[0, 0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode])
+def test_gpu_inputs_that_require_grad_without_a_gradient_to_come(mode):
+  """Parameters used under no_grad: the call is the same as with inputs that require no gradient, shares included."""
+  q, k, v = (torch.randn(1, 2, n, 128, generator=torch.Generator().manual_seed(n)).to(torch.bfloat16).to(DEV) * 0.3
+             for n in (256, 4096, 4096))
+  kernel = sa.make_splash_mha(sa.CausalMask((256, 4096), offset=4096 - 256))
+  plain, with_lse = kernel(q, k, v), kernel(q, k, v, save_residuals=True)[0]
+  leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+  with mode():
+    out = kernel(*leaves)
+  assert not out.requires_grad
+  assert torch.equal(out, plain) and torch.equal(out, with_lse)
