@@ -53,6 +53,8 @@ class BlockSizes:
     tiles.  block_q 256 selects the two-tile ping-pong forward; None picks it
     per call where it is faster.
   num_stages: depth of the forward K/V shared-memory ring.
+    With block_q, block_kv and num_stages all given every call runs that tiling
+    with one CTA per q tile, and a unit's bits do not depend on the call.
   block_kv_dq / block_q_dkv: contraction sub-block of the dQ / dK-dV kernels
     (64 or 128; None picks the largest that fits).
   num_stages_bwd: ring depth of the backward kernels.

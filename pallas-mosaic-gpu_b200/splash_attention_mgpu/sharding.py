@@ -57,6 +57,8 @@ def run_local(fn, q, k, v, segment_ids=None, *, world: int, rank: int):
 
   `fn` is a SplashAttentionKernel built with a shared (single-head) mask, or any
   callable with that signature.  Returns (local_out [units, G, S, Dv], (lo, hi)).
+  Without gradients to come the units have the bits of the whole call only where `fn`
+  was made with its forward tiling in full; to rounding they agree always.
   """
   ql, kl, vl, seg, span = local_units(q, k, v, segment_ids, world, rank)
   if ql.shape[0] == 0:

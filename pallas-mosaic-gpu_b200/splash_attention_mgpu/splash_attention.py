@@ -238,6 +238,16 @@ class SplashAttentionKernel:
   `None` fields of `block_sizes` are chosen per call from the head dims, the
   mask and the budgets; schedules are built lazily per tiling and per device,
   the backward schedule only when a gradient is first requested.
+
+  Which calls give a (batch, head) unit the same bits.  Calls that gradients follow
+  (grad mode on, an input requires grad) do, in any batch and alone.  The others may
+  choose the tiling by how much is in the call and let several CTAs share a q tile, so
+  that there a unit's result depends to rounding on the number of units beside it, and
+  differs to rounding from the one that gradients follow -- also between the first pass
+  of a reentrant checkpoint and its recomputation, or between a sharded call without
+  gradients and the whole one.  A kernel object made with a forward tiling in full
+  (block_q, block_kv and num_stages) runs that tiling with one CTA per tile in every
+  call: the same bits throughout.
   """
 
   def __init__(self, mask, *, is_mqa: bool, block_sizes: BlockSizes,
@@ -364,6 +374,12 @@ class SplashAttentionKernel:
   def block_sizes(self) -> BlockSizes:
     return self.requested_block_sizes
 
+  @property
+  def _tiling_given(self) -> bool:
+    """The caller fixed the whole forward tiling, and with it the bits: it runs as given, without shares."""
+    bs = self.requested_block_sizes
+    return None not in (bs.block_q, bs.block_kv, bs.num_stages)
+
   # -- device schedules ------------------------------------------------------
   def _fwd_schedule(self, bs: BlockSizes, device) -> _DeviceSchedule:
     key = ("fwd", bs.block_q, bs.block_kv, device.type, device.index)
@@ -437,7 +453,7 @@ def _splash_attention(kernel: SplashAttentionKernel, bs: BlockSizes, q, k, v,
     segment_ids = SegmentIds(_as_segment_tensor(seg_q, q.shape[0], q.device),
                              _as_segment_tensor(seg_kv, q.shape[0], q.device))
   if save_residuals:
-    out, lse = _forward(kernel, bs, q, k, v, segment_ids, save_residuals=True, shared_tiles=True)
+    out, lse = _forward(kernel, bs, q, k, v, segment_ids, save_residuals=True, shared_tiles=not kernel._tiling_given)
   else:
     seg_q = segment_ids.q if segment_ids is not None else None
     seg_kv = segment_ids.kv if segment_ids is not None else None
@@ -700,7 +716,7 @@ class _SplashAttentionFn(torch.autograd.Function):
   def forward(ctx, q, k, v, seg_q, seg_kv, kernel, bs, needs_grad):
     segment_ids = None if seg_q is None else SegmentIds(seg_q, seg_kv)
     out, lse = _forward(kernel, bs, q, k, v, segment_ids,
-                        save_residuals=needs_grad, shared_tiles=not needs_grad)
+                        save_residuals=needs_grad, shared_tiles=not (needs_grad or kernel._tiling_given))
     if needs_grad:
       ctx.save_for_backward(q, k, v, out, lse, *(() if seg_q is None else (seg_q, seg_kv)))
       ctx.kernel, ctx.bs = kernel, bs

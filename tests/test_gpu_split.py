@@ -142,3 +142,18 @@ def test_gpu_inputs_that_require_grad_without_a_gradient_to_come(mode):
     out = kernel(*leaves)
   assert not out.requires_grad
   assert torch.equal(out, plain) and torch.equal(out, with_lse)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,bq,bkv", [(64, 128, 64), (128, 128, 128), (128, 256, 64)])
+def test_gpu_tiling_given_in_full_keeps_a_units_bits(d, bq, bkv):
+  """Few tiles, long rows: alone, in a batch, with and without gradients, and with the logsumexp."""
+  g = lambda n: torch.randn(2, 4, n, d, generator=torch.Generator().manual_seed(n)).to(torch.bfloat16).to(DEV) * 0.3
+  q, k, v = g(256), g(4096), g(4097)[:, :, 1:].contiguous()
+  kernel = sa.make_splash_mha(sa.CausalMask((256, 4096), offset=4096 - 256),
+                              block_sizes=sa.BlockSizes(block_q=bq, block_kv=bkv, num_stages=2))
+  unit = [t[1:, 2:3] for t in (q, k, v)]
+  whole, alone, (with_lse, _) = kernel(q, k, v), kernel(*unit), kernel(*unit, save_residuals=True)
+  trained = kernel(*(t.clone().requires_grad_(True) for t in unit)).detach()
+  for x in (alone, with_lse, trained):
+    assert torch.equal(x[0, 0], whole[1, 2])
