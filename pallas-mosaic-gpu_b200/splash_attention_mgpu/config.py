@@ -5,7 +5,7 @@ messages of the reference (`splash_attention_mgpu/kernel.py:59-109`) because
 callers construct them by keyword and tests match on the error text.  The
 budget functions restate the reference's shared-memory / tensor-memory
 formulas (`kernel.py:175-189`, `forward_pingpong.py:117-128,167`,
-`backward.py:53-63,112-121,415-423`, `backward_fused.py:45-61`) so that a
+`backward.py:53-63,112-121,415-423`) so that a
 configuration the reference rejects is rejected here with the same exception
 type and wording.
 """
@@ -57,7 +57,7 @@ class BlockSizes:
     with one CTA per q tile, and a unit's bits do not depend on the call.
   block_kv_dq / block_q_dkv: contraction sub-block of the dQ / dK-dV kernels
     (64 or 128; None picks the largest that fits).
-  num_stages_bwd: ring depth of the backward kernels.
+  num_stages_bwd: ring depth of the split backward kernels (the fused one's is fixed).
   """
 
   block_q: int | None = None
@@ -159,36 +159,19 @@ def bwd_dkv_smem_bytes(*, head_dim, head_dim_v, sub_block, num_stages,
 
 
 def fused_supported(head_dim: int, head_dim_v: int) -> bool:
+  """What the fused backward needs.  Its shared-memory layout is fixed: a ring of two
+  Q tiles whatever num_stages_bwd is, and the bits of a dense mask are read from
+  global memory."""
   return head_dim == head_dim_v and head_dim in (64, 128)
 
 
-def fused_sub_block(head_dim: int) -> int:
-  """q rows per step of the fused backward (64 at either head dim)."""
-  del head_dim
-  return 64
-
-
-def fused_tmem_cols(head_dim: int) -> int:
-  """Two S^T and two dP^T buffers of 64 columns, dK and dV."""
-  return 4 * fused_sub_block(head_dim) + 2 * head_dim
-
-
-def fused_smem_bytes(*, head_dim, num_stages, itemsize, has_dense_mask,
-                     has_segments) -> int:
-  bc = fused_sub_block(head_dim)
-  bkv = TILE_ROWS
-  return (bkv * 2 * head_dim * itemsize  # K, V resident
-          + (bkv * 128 if head_dim == 64 else 0)  # second copy of K for the dQ operand
-          + num_stages * bc * 2 * head_dim * itemsize  # Q, dO ring
-          + num_stages * 2 * bc * 4  # lse, delta
-          + 2 * bkv * bc * itemsize  # dS^T staged as an MMA operand, 2 buffers
-          + 128 * 32 * 4  # dQ^T staging for the reduce-add
-          + (num_stages * bkv * bc if has_dense_mask else 0)
-          + (bkv + num_stages * bc) * 4 * bool(has_segments))
-
-
-def fused_fits(**kw) -> bool:
-  return fused_smem_bytes(**kw) <= SMEM_BYTES
+def bwd_ring_fits(*, num_stages, block_kv_dq, **kw) -> bool:
+  """Which num_stages_bwd the fused backward takes, although its own ring does not follow it: what the split
+  kernels hold at 64 rows a step, and with an explicit 128-key step of dQ one stage more than they hold there.
+  A ring beyond that is left to the split kernels, which refuse it."""
+  fits = lambda fn, sub_block, stages: fn(sub_block=sub_block, num_stages=stages, **kw) <= SMEM_BYTES
+  return (fits(bwd_dq_smem_bytes, 64, num_stages) and fits(bwd_dkv_smem_bytes, 64, num_stages)
+          and (block_kv_dq != 128 or fits(bwd_dq_smem_bytes, 128, num_stages - 1)))
 
 
 def largest_fitting_sub_block(tmem_fn, smem_fn) -> int | None:

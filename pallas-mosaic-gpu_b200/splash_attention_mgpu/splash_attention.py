@@ -614,9 +614,9 @@ def _use_fused_backward(q, v, bs: BlockSizes, has_dense, has_segments) -> bool:
                             and os.environ.get("SPLASH_BWD_FUSED_D64", "1") == "1")
   return bool(
       use and cfg.fused_supported(head_dim, v.shape[-1])
-      and cfg.fused_fits(head_dim=head_dim, num_stages=bs.num_stages_bwd,
-                         itemsize=q.element_size(), has_dense_mask=has_dense,
-                         has_segments=has_segments)
+      and cfg.bwd_ring_fits(num_stages=bs.num_stages_bwd, block_kv_dq=bs.block_kv_dq,
+                            head_dim=head_dim, head_dim_v=v.shape[-1], itemsize=q.element_size(),
+                            has_dense_mask=has_dense, has_segments=has_segments)
       and os.environ.get("SPLASH_BWD_FUSED", "1") == "1")
 
 

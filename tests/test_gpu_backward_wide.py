@@ -8,11 +8,10 @@ import torch
 
 import splash_attention_mgpu as sa
 from oracle import dense_attention as oracle
+from splash_attention_mgpu import splash_attention
 
 from common import build_mask, inputs
 from test_gpu_backward import _check_grads, _id
-
-pytestmark = pytest.mark.gpu
 
 CASES = [
     dict(mask_name="dense", s=128, d=64),                                   # one step
@@ -25,12 +24,14 @@ CASES = [
 ]
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("kwargs", CASES, ids=_id)
 def test_gpu_wide_backward(kwargs):
   kwargs = dict(kwargs)
   _check_grads(kwargs.pop("mask_name"), scaled=True, **kwargs)
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("mask_name,cap,h,kvh", [("dense", None, 2, 2), ("causal", None, 2, 2), ("full", 20.0, 4, 2)])
 def test_gpu_f16_delta_beyond_the_range_of_f16(mask_name, cap, h, kvh):
   """Loss-scaled f16 gradients: rows whose delta = dO . O is above 65504 while every operand and gradient is
@@ -54,3 +55,21 @@ def test_gpu_f16_delta_beyond_the_range_of_f16(mask_name, cap, h, kvh):
     assert np.isfinite(x).all(), name
     assert np.abs(x - r).max() / np.abs(r).max() < 2e-2, name
     assert np.abs(x - r).mean() / np.abs(r).mean() <= 1e-2, name
+
+
+def _takes_fused(d, dense, stages, **bs):
+  q = torch.empty(1, 2, 128, d, dtype=torch.bfloat16)
+  return splash_attention._use_fused_backward(q, q, sa.BlockSizes(num_stages_bwd=stages, **bs), dense, False)
+
+
+def test_ring_depth_does_not_choose_the_backward():
+  """CPU: the fused kernel's layout is fixed, so the depths that the split kernels hold run in it."""
+  assert all(_takes_fused(d, dense, n) for d in (64, 128) for dense in (False, True) for n in (1, 2, 3))
+  assert _takes_fused(128, False, 4) and not _takes_fused(128, True, 4)  # the latter is refused by the split kernels
+  assert _takes_fused(128, False, 3, block_kv_dq=128) and not _takes_fused(128, True, 3, block_kv_dq=128)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mask_name,stages", [("dense", 3), ("causal", 4)])
+def test_gpu_deep_rings(mask_name, stages):
+  _check_grads(mask_name, s=640, d=128, h=4, kvh=2, scaled=True, block_sizes=sa.BlockSizes(num_stages_bwd=stages))
