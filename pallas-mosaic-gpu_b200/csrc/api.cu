@@ -1,6 +1,7 @@
 // extern "C" entry points of libsplash_sm100.so: argument validation, dispatch to
 // the compiled kernel configuration, status helpers.
 #include "dispatch.h"
+#include "fwd_launch.cuh"
 #include "host_common.cuh"
 
 namespace splash {
@@ -87,13 +88,32 @@ extern "C" int splash_fwd256(const SplashParams* p, void* stream) {
   return fwd256(p, 1, nullptr, static_cast<cudaStream_t>(stream));
 }
 
+// Whether two CTAs of the one-tile kernel share an SM: built for it at 64-wide blocks and head dims up to 128, and
+// their shared memory fits (two stages at head_dim 128, five at 64).
+template <int D, int DV>
+static bool fwd_two_fit(const SplashParams& p) {
+  using L = FwdLayout<D, DV, 64, 1, fwd_softmax_groups<DV, 64, 1>()>;
+  const int list_steps = p.seg_q && p.seg_ranges ? p.max_steps : 0;
+  const size_t smem = L::smem_bytes(p.num_stages, p.partial_blocks != nullptr, p.seg_q != nullptr, list_steps);
+  return L::kCtasPerSm == 2 && 2 * (smem + kSmemPerCtaReserved) <= kSmemPerSm;
+}
+
+static bool fwd_two_per_sm(const SplashParams& p) {
+  if (p.block_q != 128 || p.block_kv != 64) return false;
+  if (p.head_dim == 64 && p.head_dim_v == 64) return fwd_two_fit<64, 64>(p);
+  if (p.head_dim == 64 && p.head_dim_v == 128) return fwd_two_fit<64, 128>(p);
+  if (p.head_dim == 128 && p.head_dim_v == 64) return fwd_two_fit<128, 64>(p);
+  return p.head_dim == 128 && p.head_dim_v == 128 && fwd_two_fit<128, 128>(p);
+}
+
 // CTAs per q tile that fill the GPU once.  A grid of one CTA per tile leaves SMs idle when tiles are few
 // (a chunk of queries against a long cache, small batches), and the heaviest tile then sets the time.
 // Shares of fewer than 512 keys are not made, and at least 2048 keys have to come off the longest tile:
-// the combining pass and its launch cost what about that many do.
+// the combining pass and its launch cost what about that many do.  Scheduled steps count, not those that segment ids
+// leave (1 head, 4096 tokens, D = 128, GPU time: documents of 256-4096 tokens 66.9 -> 21.5 us, of 64-256 13.7 -> 15.5).
 static int fwd_splits(const SplashParams* p) {
   if (!p || p->block_q <= 0 || p->q_len <= 0 || p->batch <= 0 || p->heads <= 0) return 1;
-  const bool two_per_sm = p->block_q == 128 && p->block_kv == 64 && p->head_dim <= 128 && p->head_dim_v <= 128;
+  const bool two_per_sm = fwd_two_per_sm(*p);
   const int64_t slots = static_cast<int64_t>(sm_count()) * (two_per_sm ? 2 : 1);
   const int64_t tiles = static_cast<int64_t>(p->q_len / p->block_q) * p->heads * p->batch;
   if (tiles <= 0) return 1;

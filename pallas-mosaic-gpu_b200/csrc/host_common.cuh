@@ -106,5 +106,6 @@ inline int sm_count() {
 }
 
 constexpr size_t kMaxDynamicSmem = 227 * 1024;
+constexpr size_t kSmemPerSm = 228 * 1024, kSmemPerCtaReserved = 1024;
 
 }  // namespace splash

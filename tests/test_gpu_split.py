@@ -38,6 +38,15 @@ def test_forward_share_rule():
   assert size(heads=1, q_len=128, kv_len=1 << 20, max_steps=1 << 13) == 32 * rows(1, 128)
 
 
+def test_forward_shares_count_the_ctas_that_an_sm_holds():
+  """CPU: 128 tiles of 64-wide blocks get a second CTA each only where two CTAs' shared memory fits an SM."""
+  size = lambda d, stages, **kw: _ffi.load().splash_fwd_split_bytes(ctypes.byref(_params(
+      heads=32, q_len=512, block_kv=64, max_steps=128, **dict(dict(head_dim=d, head_dim_v=d, num_stages=stages), **kw))))
+  assert size(128, 2) > 0 and size(128, 3) == 0
+  assert size(64, 5) > 0 and size(64, 6) == 0
+  assert size(128, 2, head_dim_v=64) > 0 and size(192, 2) == 0
+
+
 def test_tiling_of_few_tiles():
   """CPU: 128-wide blocks for up to one tile per SM, up to 7/4 where row lengths differ; a tiling of which
   a part is given stays what it was."""
