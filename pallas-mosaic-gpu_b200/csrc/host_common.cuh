@@ -9,6 +9,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -95,13 +96,15 @@ inline int opt_in_smem(Kernel kernel, size_t bytes) {
   return opt_in_smem_impl(reinterpret_cast<const void*>(kernel), bytes);
 }
 
-// SMs of the current device (the library is built for one GPU model: asked once).
+// SMs of the current device, asked once per device; those of a B200 where there is none to ask.
 inline int sm_count() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
-    return v;
-  }();
+  constexpr int kB200Sms = 148, kDevices = 64;
+  static std::atomic<int> known[kDevices];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return kB200Sms;
+  if ((n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return kB200Sms;
+  known[dev].store(n, std::memory_order_relaxed);
   return n;
 }
 

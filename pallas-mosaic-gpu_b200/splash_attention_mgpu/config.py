@@ -22,7 +22,7 @@ DEFAULT_MASK_VALUE = -0.7 * float(np.finfo(np.dtype("float32")).max)
 TILE_ROWS = 128  # query rows handled by one softmax warpgroup (one TMEM lane each)
 PINGPONG_ROWS = 2 * TILE_ROWS
 TMEM_COLS = 512
-NUM_SMS = 148
+NUM_SMS = 148  # of a B200, the one GPU the kernels are built for; the library asks the device for its shares
 # Bounds on a call's number of 128-row q tiles: up to one per SM, up to one and three quarters.
 FEW_TILES = (NUM_SMS, NUM_SMS * 7 // 4)
 # 227 KiB of dynamic shared memory per CTA on sm_100, minus room for barriers

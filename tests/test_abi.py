@@ -5,6 +5,10 @@ No compute calls are made here."""
 import ctypes
 import os
 import re
+import shutil
+import subprocess
+
+import pytest
 
 from splash_attention_mgpu import _ffi
 
@@ -52,3 +56,37 @@ def test_status_strings_and_argument_checks_need_no_gpu():
   assert b"non-null" in lib.splash_last_error()
   assert lib.splash_bwd_fused(ctypes.byref(p), None) == _ffi.SPLASH_INVALID_ARGUMENT
   assert lib.splash_selftest_umma(None, None, None, 128, 128, 0, 0, 0, None, None) == _ffi.SPLASH_INVALID_ARGUMENT
+
+
+def test_sm_count_is_asked_per_device(tmp_path):
+  """The host helper behind the shares of a q tile, against a stand-in for the runtime with two devices."""
+  cuda = "/usr/local/cuda/include"
+  if shutil.which("g++") is None or not os.path.isdir(cuda):
+    pytest.skip("needs g++ and the CUDA headers")
+  (tmp_path / "main.cpp").write_text('''
+#include "host_common.cuh"
+static int device = 0, answers = 0;
+extern "C" cudaError_t cudaGetDevice(int* d) { *d = device; return device < 0 ? cudaErrorNoDevice : cudaSuccess; }
+extern "C" cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int d) {
+  ++answers;
+  if (d == 2) return cudaErrorInvalidDevice;
+  *v = d == 0 ? 148 : 132;
+  return cudaSuccess;
+}
+int main() {
+  device = -1;                                     // nobody to ask: not remembered
+  if (splash::sm_count() != 148) return 1;
+  device = 2;
+  if (splash::sm_count() != 148) return 2;
+  device = 1;
+  if (splash::sm_count() != 132) return 3;
+  device = 0;
+  if (splash::sm_count() != 148) return 4;
+  device = 1;
+  return splash::sm_count() == 132 && answers == 3 ? 0 : 5;
+}
+''')
+  exe = tmp_path / "main"
+  subprocess.run(["g++", "-std=c++17", "-w", "-O1", "-I", cuda, "-I", os.path.join(ROOT, "pallas-mosaic-gpu_b200", "csrc"),
+                  str(tmp_path / "main.cpp"), "-o", str(exe)], check=True)
+  assert subprocess.run([str(exe)]).returncode == 0
