@@ -282,6 +282,18 @@ class SplashAttentionKernel:
     return (float(self.fwd_info(256, 128).num_steps.sum()) * 256
             / max(1.0, float(self.fwd_info(128, 128).num_steps.sum()) * 128))
 
+  @property
+  def _short_rows(self) -> bool:
+    """Rows too short for 128-wide blocks to pay: one block, or up to three of a longer sequence, or four of which
+    64-wide ones need clearly fewer keys (a window that is no multiple of 128)."""
+    info = self.fwd_info(128, 128)
+    steps = int(info.num_steps.max())
+    if steps <= 1:
+      return True
+    if steps > 4 or steps >= self.mask.shape[-1] // 128 or info.partial_mask_blocks is not None:
+      return False
+    return steps <= 3 or int(info.num_steps.sum()) * 128 > 1.1 * int(self.fwd_info(128, 64).num_steps.sum()) * 64
+
   def _auto_forward_tiling(self, head_dim: int, head_dim_v: int, *,
                            itemsize: int = 2, has_segments: bool = False,
                            save_residuals: bool = True,
@@ -298,14 +310,21 @@ class SplashAttentionKernel:
 
     `tiles` is the call's number of 128-row q tiles over batch and heads.  Up to one per SM the second
     CTA that 64-wide blocks leave room for has no tile, and 128-wide blocks with their two softmax
-    warpgroups are faster at any row length (causal, D = 128: 8 heads, seq 1024 21.3 -> 18.4 us, 4 heads,
+    warpgroups are faster from rows of a few blocks on (causal, D = 128: 8 heads, seq 1024 21.3 -> 18.4 us, 4 heads,
     seq 4096 53 -> 38 us; D = 64: 2 heads, seq 4096 49 -> 37 us).  Up to one and three quarters per SM that
     still holds where the rows differ in length as under a causal mask, for the two CTAs that share an SM
     then hold up its longest row (192 tiles, seq 2048: 36.9 -> 28.7 us; 256 tiles, seq 4096: 59 -> 44 us; at
     288 tiles 41.0 against 41.8), but not where they are alike (local, 192 tiles: 23.5 against 26.6 us).
+    Segment ids can make rows shorter than the mask says (256 tiles, seq 2048, causal, D = 128: documents of
+    256-4096 tokens 35.2 -> 29.5 us, of 64-1024 24.5 against 26.1).
+
+    Short rows keep their tiling (GPU time, 128-wide over 64-wide blocks, 128 tiles, seq 2048 and 8192): a
+    single block (seq 128: 5.9 against 7.0 us), and windows or chunks of few blocks, where the wide ones visit keys
+    that the narrow ones do not or the groups hardly alternate (window 64 1.17, 128 1.02, 256 1.07, 320 1.06,
+    384 1.00, 512 0.96; chunks of 256 1.04, of 384 1.02, of 512 0.94).
     """
     if (tiles is not None and head_dim == head_dim_v and head_dim in (64, 128)
-        and tiles <= cfg.FEW_TILES[1]):
+        and tiles <= cfg.FEW_TILES[1] and not self._short_rows):
       info = self.fwd_info(128, 128)
       few = dict(head_dim=head_dim, head_dim_v=head_dim_v, block_kv=128, num_stages=2, itemsize=itemsize,
                  has_dense_mask=info.partial_mask_blocks is not None,

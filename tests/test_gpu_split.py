@@ -52,13 +52,26 @@ def test_tiling_of_few_tiles():
   a part is given stays what it was."""
   tiling = lambda mask, tiles, d=128, **bs: (lambda r: (r.block_q, r.block_kv, r.num_stages))(
       sa.make_splash_mha(mask, block_sizes=sa.BlockSizes(**bs)).resolved_block_sizes(d, d, tiles=tiles))
-  causal, local = sa.CausalMask((1024, 1024)), sa.LocalMask((2048, 2048), (256, 0), 0)
+  causal, local = sa.CausalMask((1024, 1024)), sa.LocalMask((2048, 2048), (512, 0), 0)
   for d in (64, 128):
     assert tiling(causal, 148, d) == (128, 128, 2) == tiling(causal, 259, d)
     assert tiling(causal, 260, d) == tiling(causal, None, d) == (128, 64, 2)
     assert tiling(local, 148, d) == (128, 128, 2) and tiling(local, 149, d) == (128, 64, 2)
   assert tiling(causal, 8, block_kv=64) == (128, 64, 2) == tiling(causal, None, block_kv=64)
   assert tiling(causal, 8, num_stages=3) == (128, 64, 3)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_short_rows_keep_their_tiling(d):
+  """CPU: few tiles, but a single block a row or a narrow window: the tiling that does not depend on the call."""
+  tiling = lambda mask, tiles: (lambda r: (r.block_q, r.block_kv, r.num_stages))(
+      sa.make_splash_mha(mask).resolved_block_sizes(d, d, tiles=tiles))
+  window = lambda w: sa.LocalMask((2048, 2048), (w, 0), 0)
+  chunks = lambda c: sa.ChunkedCausalMask((2048, 2048), chunk_size=c)
+  for mask in [sa.CausalMask((128, 128)), *map(window, (64, 128, 256, 320)), *map(chunks, (128, 256, 384))]:
+    assert tiling(mask, 8) == tiling(mask, None) == (128, 64, 2)
+  for mask in [sa.CausalMask((256, 256)), sa.CausalMask((384, 384)), window(384), window(512), chunks(512)]:
+    assert tiling(mask, 8) == (128, 128, 2) != tiling(mask, None)
 
 
 CASES = [
