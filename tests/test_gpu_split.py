@@ -12,7 +12,7 @@ import splash_attention_mgpu as sa
 from oracle import dense_attention as oracle
 from splash_attention_mgpu import _ffi
 
-from common import assert_forward_close
+from common import assert_forward_close, inputs
 
 DEV = "cuda:0"
 
@@ -179,3 +179,44 @@ def test_gpu_tiling_given_in_full_keeps_a_units_bits(d, bq, bkv):
   trained = kernel(*(t.clone().requires_grad_(True) for t in unit)).detach()
   for x in (alone, with_lse, trained):
     assert torch.equal(x[0, 0], whole[1, 2])
+
+
+def _local(q, kv, window):
+  return sa.LocalMask((q, kv), (window, 0), kv - q)
+
+
+FORMS = [
+    dict(mask=lambda q, kv: sa.CausalMask((q, kv), offset=kv - q), d=192),
+    dict(mask=lambda q, kv: sa.CausalMask((q, kv), offset=kv - q), d=128, dv=64),
+    dict(mask=lambda q, kv: sa.CausalMask((q, kv), offset=kv - q), d=64, dv=128, cap=10.0),
+    dict(mask=lambda q, kv: _local(q, kv, 3000), kv=8192),
+    dict(mask=lambda q, kv: sa.ChunkedCausalMask((q, kv), chunk_size=3072), q=6144, kv=6144, h=1),
+    dict(mask=lambda q, kv: sa.MultiHeadMask([sa.CausalMask((q, kv), offset=kv - q), _local(q, kv, 700),
+                                              sa.FullMask((q, kv))]), h=3, d=64),
+    dict(mask=lambda q, kv: sa.CausalMask((q, kv), offset=kv - q), h=3, mqa=True, dtype=torch.float16),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c", FORMS, ids=["d192", "d128-dv64", "d64-dv128-cap", "local", "chunked", "per-head", "mqa"])
+def test_gpu_shares_by_plain_inference(c, monkeypatch):
+  """The call that writes no logsumexp, for the masks and head dims that the cases above leave out: it takes shares,
+  agrees with the oracle, and has the bits of the call with a logsumexp."""
+  q_len, kv_len, h, d = c.get("q", 256), c.get("kv", 4096), c.get("h", 2), c.get("d", 128)
+  dtype, cap, mqa = c.get("dtype", torch.bfloat16), c.get("cap"), c.get("mqa", False)
+  mask = c["mask"](q_len, kv_len)
+  heads = mask.masks if isinstance(mask, sa.MultiHeadMask) else [mask]
+  dense = np.stack([np.asarray(m[:, :]) for m in heads])
+  q, k, v = inputs(1, h, h, kv_len, d, c.get("dv", d), dtype, mqa, seed=2, device=DEV)
+  q = (q[:, :, :q_len] * d ** -0.5).contiguous()
+  kernel = (sa.make_splash_mqa if mqa else sa.make_splash_mha)(mask, attn_logits_soft_cap=cap)
+  lib, shared = _ffi.load(), []
+  entry = lib.splash_fwd_split
+  monkeypatch.setattr(lib, "splash_fwd_split", lambda *a: shared.append(entry(*a)) or shared[-1])
+  out = kernel(q, k, v)
+  assert shared == [0]
+  with_lse, (lse,) = kernel(q, k, v, save_residuals=True)
+  sa.check_device_status()
+  assert shared == [0, 0] and torch.equal(out, with_lse)
+  ref, ref_lse = oracle.attention_forward(dense, q, k, v, is_mqa=mqa, attn_logits_soft_cap=cap)
+  assert_forward_close(out, lse, ref, ref_lse, dtype)
