@@ -186,7 +186,7 @@ def _local(q, kv, window):
 
 
 FORMS = [
-    dict(mask=lambda q, kv: sa.CausalMask((q, kv), offset=kv - q), d=192),
+    dict(mask=lambda q, kv: sa.CausalMask((q, kv), offset=kv - q), d=192, block_sizes=sa.BlockSizes(block_kv=64)),
     dict(mask=lambda q, kv: sa.CausalMask((q, kv), offset=kv - q), d=128, dv=64),
     dict(mask=lambda q, kv: sa.CausalMask((q, kv), offset=kv - q), d=64, dv=128, cap=10.0),
     dict(mask=lambda q, kv: _local(q, kv, 3000), kv=8192),
@@ -209,7 +209,8 @@ def test_gpu_shares_by_plain_inference(c, monkeypatch):
   dense = np.stack([np.asarray(m[:, :]) for m in heads])
   q, k, v = inputs(1, h, h, kv_len, d, c.get("dv", d), dtype, mqa, seed=2, device=DEV)
   q = (q[:, :, :q_len] * d ** -0.5).contiguous()
-  kernel = (sa.make_splash_mqa if mqa else sa.make_splash_mha)(mask, attn_logits_soft_cap=cap)
+  kernel = (sa.make_splash_mqa if mqa else sa.make_splash_mha)(mask, block_sizes=c.get("block_sizes"),
+                                                               attn_logits_soft_cap=cap)
   lib, shared = _ffi.load(), []
   entry = lib.splash_fwd_split
   monkeypatch.setattr(lib, "splash_fwd_split", lambda *a: shared.append(entry(*a)) or shared[-1])
