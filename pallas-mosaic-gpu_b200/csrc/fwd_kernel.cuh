@@ -7,7 +7,7 @@
 //           a two-stage ring two such CTAs share an SM.
 //   NT = 1, AW = 2  the same tile with two softmax warpgroups that take the KV steps
 //           in turn (128-wide KV blocks; 64-wide ones at head_dim_v 64, still two CTAs
-//           per SM, and above 128).  The groups hand the stale row maximum to
+//           per SM, and above 128, unless rows are short).  The groups hand the stale row maximum to
 //           one another through shared memory, keep partial row sums and split the
 //           epilogue; P has tensor-memory columns of its own, so the S buffer of step
 //           s is free as soon as its softmax has read it and Q.K^T of step s+2 runs

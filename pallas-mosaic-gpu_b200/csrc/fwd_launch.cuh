@@ -81,14 +81,17 @@ int launch_fwd_plain(const SplashParams& p, int splits, void* workspace, cudaStr
 }
 
 // The kernel without its soft-cap, segment and streamed-mask code when the call uses none.
+template <int D, int DV, int BKV, int NT, int AW, bool SPLIT, bool BF16>
+int launch_fwd_form(const SplashParams& p, int splits, void* workspace, cudaStream_t stream) {
+  const bool plain = p.soft_cap == 0.f && p.seg_q == nullptr && p.partial_blocks == nullptr;
+  return plain ? launch_fwd_plain<D, DV, BKV, NT, AW, true, SPLIT, BF16>(p, splits, workspace, stream)
+               : launch_fwd_plain<D, DV, BKV, NT, AW, false, SPLIT, BF16>(p, splits, workspace, stream);
+}
+
 template <int D, int DV, int BKV, int NT, int AW, bool BF16>
 int launch_fwd_typed(const SplashParams& p, int splits, void* workspace, cudaStream_t stream) {
-  const bool plain = p.soft_cap == 0.f && p.seg_q == nullptr && p.partial_blocks == nullptr;
-  if (splits > 1)
-    return plain ? launch_fwd_plain<D, DV, BKV, NT, AW, true, true, BF16>(p, splits, workspace, stream)
-                 : launch_fwd_plain<D, DV, BKV, NT, AW, false, true, BF16>(p, splits, workspace, stream);
-  return plain ? launch_fwd_plain<D, DV, BKV, NT, AW, true, false, BF16>(p, splits, workspace, stream)
-               : launch_fwd_plain<D, DV, BKV, NT, AW, false, false, BF16>(p, splits, workspace, stream);
+  return splits > 1 ? launch_fwd_form<D, DV, BKV, NT, AW, true, BF16>(p, splits, workspace, stream)
+                    : launch_fwd_form<D, DV, BKV, NT, AW, false, BF16>(p, splits, workspace, stream);
 }
 
 // Softmax warpgroups per q tile of the one-tile kernel.  Two that alternate over the KV steps where
@@ -105,10 +108,27 @@ constexpr int fwd_softmax_groups() {
   return 3 * BKV + DV <= 512 ? 2 : 1;
 }
 
+// Rows of few steps, where two groups hardly take turns and their hand-over and larger start only cost: one group.
+// Up to head_dim 128 by the longest row (one group against two, bf16, seq 8192, D = 64, 64 heads: window 64, 3 steps,
+// 101.7 against 108.0 us, window 256, 6 steps, 136.5 / 137.5, window 512, 10 steps, 178.4 / 171.8; batch 32, 16 heads, seq
+// 128 13.1 / 14.7; batch 16, seq 512 33.8 / 34.4).  Above it, where one CTA has the SM, where a row spans all keys, as in
+// batches of short sequences (batch 16, 16 heads, seq 512, D = 256 full 88.5 / 96.4, causal 75.6 / 79.6; batch 8, seq 1024
+// 142.5 / 150.6, 102.0 / 108.8; D = 192 112.4 / 115.4, 85.6 / 87.4); windows are even there (+-1.5 %) and keep two.
+template <int D, int DV>
+bool fwd_short_rows(const SplashParams& p) {
+  if (D <= 128 && DV <= 128) return p.max_steps <= 8;
+  return p.max_steps <= 16 && p.max_steps * p.block_kv >= p.kv_len;
+}
+
 template <int D, int DV, int BKV, int NT>
 int launch_fwd(const SplashParams& p, int splits, void* workspace, cudaStream_t stream) {
   const bool bf16 = p.dtype == SPLASH_DTYPE_BF16;
   constexpr int AW = fwd_softmax_groups<DV, BKV, NT>();
+  if constexpr (NT == 1 && BKV == 64 && AW == 2) {
+    if (splits == 1 && fwd_short_rows<D, DV>(p))
+      return bf16 ? launch_fwd_form<D, DV, BKV, NT, 1, false, true>(p, 1, nullptr, stream)
+                  : launch_fwd_form<D, DV, BKV, NT, 1, false, false>(p, 1, nullptr, stream);
+  }
   if (bf16) return launch_fwd_typed<D, DV, BKV, NT, AW, true>(p, splits, workspace, stream);
   return launch_fwd_typed<D, DV, BKV, NT, AW, false>(p, splits, workspace, stream);
 }

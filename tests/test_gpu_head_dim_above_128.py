@@ -1,6 +1,6 @@
-"""The forward at head_dim 192 and 256 with 64-wide KV blocks, where two softmax groups take the steps in
-turn with one CTA per SM: the fewest steps (one of the groups without a step of its own), odd counts, every
-masking option; against the CPU oracle with the bars of test_gpu_forward.py."""
+"""The forward at head_dim 192 and 256 with 64-wide KV blocks, one softmax group where rows of up to 16 steps span
+all keys, else two that take the steps in turn, with one CTA per SM: the fewest steps, odd counts, every
+masking option (rows of two steps beside long ones in two groups: test_gpu_short_rows.py); against the CPU oracle with the bars of test_gpu_forward.py."""
 
 import numpy as np
 import pytest
