@@ -169,6 +169,8 @@ def bwd_ring_fits(*, num_stages, block_kv_dq, **kw) -> bool:
   """Which num_stages_bwd the fused backward takes, although its own ring does not follow it: what the split
   kernels hold at 64 rows a step, and with an explicit 128-key step of dQ one stage more than they hold there.
   A ring beyond that is left to the split kernels, which refuse it."""
+  if num_stages <= 2:  # fits whatever the call; this is asked for every backward
+    return True
   fits = lambda fn, sub_block, stages: fn(sub_block=sub_block, num_stages=stages, **kw) <= SMEM_BYTES
   return (fits(bwd_dq_smem_bytes, 64, num_stages) and fits(bwd_dkv_smem_bytes, 64, num_stages)
           and (block_kv_dq != 128 or fits(bwd_dq_smem_bytes, 128, num_stages - 1)))
