@@ -113,11 +113,11 @@ static bool fwd_two_per_sm(const SplashParams& p) {
 // leave (1 head, 4096 tokens, D = 128, GPU time: documents of 256-4096 tokens 66.9 -> 21.5 us, of 64-256 13.7 -> 15.5).
 static int fwd_splits(const SplashParams* p) {
   if (!p || p->block_q <= 0 || p->q_len <= 0 || p->batch <= 0 || p->heads <= 0) return 1;
-  const bool two_per_sm = fwd_two_per_sm(*p);
-  const int64_t slots = static_cast<int64_t>(sm_count()) * (two_per_sm ? 2 : 1);
+  const int64_t keys = static_cast<int64_t>(p->max_steps) * p->block_kv;
+  if (keys <= 2048) return 1;  // (short calls, whose host time counts, ask no further)
   const int64_t tiles = static_cast<int64_t>(p->q_len / p->block_q) * p->heads * p->batch;
   if (tiles <= 0) return 1;
-  const int64_t keys = static_cast<int64_t>(p->max_steps) * p->block_kv;
+  const int64_t slots = static_cast<int64_t>(sm_count()) * (fwd_two_per_sm(*p) ? 2 : 1);
   int64_t splits = slots / tiles;
   if (splits > keys / 512) splits = keys / 512;
   if (splits > 32) splits = 32;

@@ -397,7 +397,7 @@ class SplashAttentionKernel:
   def _tiling_given(self) -> bool:
     """The caller fixed the whole forward tiling, and with it the bits: it runs as given, without shares."""
     bs = self.requested_block_sizes
-    return None not in (bs.block_q, bs.block_kv, bs.num_stages)
+    return bs.num_stages is not None and bs.block_q is not None and bs.block_kv is not None
 
   # -- device schedules ------------------------------------------------------
   def _fwd_schedule(self, bs: BlockSizes, device) -> _DeviceSchedule:
